@@ -62,7 +62,8 @@ typedef struct gs_options {
   float shLr;          /* opts.shLr, default 1.25e-4 (trainer.js:302) */
   /* B200 options (no reference counterpart) */
   int32_t tile;            /* raster tile edge in pixels: 8, 16 (the reference's TILE) or 32 */
-  int32_t batchDepth;      /* splat records staged per shared-memory batch: 64, 128 or 256 */
+  int32_t batchDepth;      /* splat records staged per shared-memory batch: 64, 128 or 256 (stored-state
+                              variant; the recomputing raster stages 32 per warp whatever the depth) */
   int32_t maxBatch;        /* most views one gs_step_batch may take (buffers are sized for it) */
   int32_t backwardVariant; /* 0: recompute transmittance from the final T (reference); 1: stored-state */
   int32_t persistent;      /* 1: raster over a persistent (view, tile) work queue, heaviest tiles first */

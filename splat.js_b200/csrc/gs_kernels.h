@@ -57,18 +57,18 @@ struct ExpandArgs {
   const DevCam* cams;
   const uint32_t* sortedSlots;  // presorted (view, depth, id) order
   const uint4* itemSrc;         // V * n * 2 by slot: (rect, mean, cull parameters, slot) from the projection
-  uint4* itemRecs;              // V * n * 2: the same per presorted item (mean and cull parameters only
-                                // when cull != 0)
+  uint4* itemRecs;              // V * n * 2: the same per presorted item
   const uint32_t* liveItems;    // presorted items kept (the culled ones left the presort)
   const uint8_t* dropped;
   const uint32_t* viewDrops;
   float eCut, aMin;
   int tile;
   int cull;                     // 1: keep only entries tileLive() accepts
+  int masks;                    // 1 (tile 16): entry values carry the 8x8 block bits
   uint32_t* counts;             // count pass: V * n, in presorted order
   const uint32_t* offsets;      // key pass: V * n exclusive scan of counts
   uint32_t* keys;               // global tile id per entry
-  uint32_t* vals;               // splat id per entry
+  uint32_t* vals;               // entry value: splat id (and block bits)
   uint64_t capacity;
   uint32_t* status;
 };
@@ -123,13 +123,26 @@ struct RadixSortArgs {
                             // across a warp: tile ids, the low bytes of depths)
 };
 
+// Entry values.  With block masks on (16-pixel tiles, at most 2^28 splats) a
+// value is the splat id in the low ID_BITS bits and, above it, one bit per 8x8
+// block of the tile (row-major): set when the splat may reach the block.
+constexpr uint32_t ID_BITS = 28;
+constexpr uint32_t ID_MASK = (1u << ID_BITS) - 1u;
+
+constexpr int RW_WARPS = 4;                    // warps per block of k_raster_warp
+#ifndef GS_RASTER_CACHE
+#define GS_RASTER_CACHE 256  // composited entries a warp caches (k_raster_warp)
+#endif
+constexpr uint32_t RASTER_CACHE_ENTRIES = GS_RASTER_CACHE;
+
 struct RasterArgs {
   const DevCam* cams;
   int V;
   uint32_t n;
   const RenderRec* recs;   // V * n
   const float4* cullRecs;  // V * n warp-block cull parameters
-  const uint32_t* ids;     // sorted entry values (splat ids)
+  const uint32_t* ids;     // sorted entry values: splat ids under idMask, block bits above it
+  uint32_t idMask;         // ID_MASK with block masks, else all ones
   const uint2* ranges;     // per global tile
   uint32_t totalTiles;
   const uint32_t* workOrder;  // null: item order
@@ -143,6 +156,10 @@ struct RasterArgs {
   uint32_t* stats;
   int32_t* gradCam;
   float* tStore;           // stored-state variant: T before each entry, per pixel
+  // k_raster_warp's exponential cache: cacheWarps slices of cacheCap + 2 entries, and one more
+  uint32_t cacheCap, cacheWarps;
+  float2* cacheG;          // per entry 32 lanes x 2 pixels
+  uint32_t* cacheId;       // per entry the splat id
 };
 
 struct AdamHP {
@@ -220,9 +237,10 @@ int export_ply_records(const float* params, const float* sh, uint32_t n, uint32_
                        cudaStream_t s);
 int debug_lookback_timeout(int device, uint32_t spinLimit, uint32_t* statusOut, double* msOut);
 void launch_radix_sort(const RadixSortArgs& a, cudaStream_t s);
-void launch_raster(const RasterArgs& a, int mode, bool stored, int tile, int batchDepth, unsigned grid,
-                   cudaStream_t s);
-int raster_blocks_per_sm(int tile, int batchDepth, int mode);
+void launch_raster(const RasterArgs& a, bool train, int tile, unsigned grid, int sms, cudaStream_t s);
+unsigned raster_grid(uint32_t items, int sms, int perSm);
+void launch_raster_stored(const RasterArgs& a, int tile, int batchDepth, unsigned grid, cudaStream_t s);
+int raster_blocks_per_sm(int tile, bool train);
 void launch_work_order(const uint2* ranges, uint32_t totalTiles, uint32_t* order, uint32_t* scratch,
                        cudaStream_t s);
 void launch_chain_adam(const ChainArgs& a, int deg, cudaStream_t s);

@@ -285,10 +285,11 @@ __global__ void k_tile_ranges_finish(TileRangeArgs a, uint32_t totalTiles) {
 // X0 and X1 non-decreasing in tx, so the live tiles of a row form one run
 // [ca, cb]; two binary searches on the same predicates find it, giving
 // exactly the tiles tileLive() accepts.  Returns the run length (0: none).
-__device__ __forceinline__ uint32_t row_run(const float4 cq, float mx, float my, uint32_t x0, uint32_t x1,
+// test = false: the whole row is kept.
+__device__ __forceinline__ uint32_t row_run(bool test, const float4 cq, float mx, float my, uint32_t x0, uint32_t x1,
                                             uint32_t ty, int tile, int W, int H, uint32_t& ca) {
   ca = x0;
-  if (!(cq.x < 3.0e38f)) return x1 - x0 + 1;
+  if (!test || !(cq.x < 3.0e38f)) return x1 - x0 + 1;
   const int ye = (int)ty * tile + tile < H ? (int)ty * tile + tile : H;
   float xl, xr;
   if (!bandInterval(cq, ((float)((int)ty * tile) + 0.5f) - my, ((float)(ye - 1) + 0.5f) - my, xl, xr)) return 0;
@@ -309,6 +310,34 @@ __device__ __forceinline__ uint32_t row_run(const float4 cq, float mx, float my,
     else hi = mid;
   }
   return lo - ca;
+}
+
+// Block columns (8 pixels wide, counted from tile column ca of a 16-pixel
+// tile row) that the splat may reach in the 8 pixel rows from y0: first | last
+// << 16, first > last when there are none, 65535 as last meaning no bound.
+// The interval is bandIntervalMask's, so conservative; the slack added here
+// covers the rounding of the shift to image coordinates.
+__device__ __forceinline__ uint32_t band_columns(const float4 cq, float mx, float my, uint32_t y0, uint32_t ca) {
+  if (!(cq.x < 3.0e38f)) return 0xFFFF0000u;
+  const float Y0 = ((float)y0 + 0.5f) - my;
+  float xl, xr;
+  if (!bandIntervalMask(cq, Y0, Y0 + 7.0f, xl, xr)) return 1u;
+  const float sl = 4.0e-6f * (fabsf(mx) + fmaxf(fabsf(xl), fabsf(xr)) + 8.0f);
+  const float base = 2.0f * (float)ca;
+  const float l = clampf(ceilf(((xl + mx) - 7.5f - sl) * 0.125f) - base, 0.0f, 65535.0f);
+  const float r = clampf(floorf(((xr + mx) - 0.5f + sl) * 0.125f) - base, -1.0f, 65535.0f);
+  if (r < 0.0f) return 1u;
+  return (uint32_t)l | ((uint32_t)r << 16);
+}
+// block bits of a tile whose left block column is col: bands b0 (rows 0-7), b1
+__device__ __forceinline__ uint32_t block_bits(uint32_t b0, uint32_t b1, uint32_t col) {
+  uint32_t m = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 4; ++k) {
+    const uint32_t b = k < 2 ? b0 : b1, c = col + (k & 1u);
+    if (c >= (b & 0xFFFFu) && (c <= (b >> 16) || (b >> 16) == 0xFFFFu)) m |= 1u << k;
+  }
+  return m << ID_BITS;
 }
 
 // Entry expansion of the presorted items, in two passes over the same walk:
@@ -356,7 +385,7 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
       slot = a.sortedSlots[p];
       const uint4 s0 = a.itemSrc[2 * slot], s1 = a.itemSrc[2 * slot + 1];
       r = make_uint2(s0.x, s0.y);
-      if (r.x != 0xFFFFFFFFu && a.cull) {
+      if (r.x != 0xFFFFFFFFu) {
         mx = __uint_as_float(s0.z); my = __uint_as_float(s0.w);
         cq = make_float4(__uint_as_float(s1.x), __uint_as_float(s1.y), __uint_as_float(s1.z), 0.0f);
       }
@@ -389,7 +418,11 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
             if (dr[t]) continue;
             if (test && !tileLive(cq, mx, my, (int)x, (int)y, a.tile, c.W, c.H)) continue;
             if (KEYS) {
-              if (o < a.capacity) { a.keys[o] = c.tileBase + t; a.vals[o] = i; }
+              if (o < a.capacity) {
+                a.keys[o] = c.tileBase + t;
+                a.vals[o] = i | (a.masks ? block_bits(band_columns(cq, mx, my, y * 16, x),
+                                                      band_columns(cq, mx, my, y * 16 + 8, x), 0u) : 0u);
+              }
               else atomicOr(a.status, ST_ENTRY_OVERFLOW);
               ++o;
             }
@@ -399,7 +432,6 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
       }
     }
   }
-  if (!test) cq = make_float4(__int_as_float(0x7F800000), 0.0f, 0.0f, 0.0f);  // untested: whole rows
   __syncwarp();
   // row offsets of the warp's items (inclusive scan of rr)
   uint32_t rEnd = rr;
@@ -424,7 +456,8 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
     const uint32_t ox0 = __shfl_sync(FULL, x0, lo);
     const uint32_t ox1 = __shfl_sync(FULL, x1, lo);
     const uint32_t oy0 = __shfl_sync(FULL, y0, lo);
-    const uint32_t ov = __shfl_sync(FULL, v, lo);
+    const uint32_t ovt = __shfl_sync(FULL, v | (test ? 0x80000000u : 0u), lo);
+    const uint32_t ov = ovt & 0x7FFFFFFFu;
     const float omx = __shfl_sync(FULL, mx, lo);
     const float omy = __shfl_sync(FULL, my, lo);
     float4 ocq;
@@ -436,7 +469,12 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
     if (inRange) {
       ty = oy0 + (u - orb);
       const DevCam& c = a.cams[ov];
-      cnt = row_run(ocq, omx, omy, ox0, ox1, ty, a.tile, c.W, c.H, ca);
+      cnt = row_run((ovt >> 31) != 0u, ocq, omx, omy, ox0, ox1, ty, a.tile, c.W, c.H, ca);
+    }
+    uint32_t band0 = 0, band1 = 0;
+    if (KEYS && a.masks && cnt) {
+      band0 = band_columns(ocq, omx, omy, ty * 16, ca);
+      band1 = band_columns(ocq, omx, omy, ty * 16 + 8, ca);
     }
     const uint32_t peers = __match_any_sync(FULL, inRange ? (uint32_t)lo : 32u);
     const int lead = __ffs(peers) - 1;
@@ -481,7 +519,11 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
         w = (k0 <= e) ? l2 : -1;
         const uint32_t wc = __shfl_sync(FULL, cnt, l2 & 31);
         const uint32_t wk = __shfl_sync(FULL, rowKey, l2 & 31);
-        const uint32_t wi = __shfl_sync(FULL, oi, l2 & 31);
+        uint32_t wi = __shfl_sync(FULL, oi, l2 & 31);
+        if (a.masks) {
+          const uint32_t w0 = __shfl_sync(FULL, band0, l2 & 31), w1 = __shfl_sync(FULL, band1, l2 & 31);
+          wi |= block_bits(w0, w1, 2u * (e - k0));
+        }
         if (w >= 0 && e < lastEnd && e - k0 < wc) {
           if (e < a.capacity) { a.keys[e] = wk + (e - k0); a.vals[e] = wi; }
           else atomicOr(a.status, ST_ENTRY_OVERFLOW);

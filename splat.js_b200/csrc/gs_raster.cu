@@ -2,30 +2,24 @@
 // the back-to-front backward of the reference's render pass
 // (shaders.js:544-700), over a shared (view, tile) work queue.
 //
-// One CTA works on one TILE x TILE tile at a time (TILE = 8, 16 or 32; one
-// thread per pixel; each warp covers an 8x4 block of the tile).  Splat
-// records of the tile's sorted entries are staged in shared memory BATCH at
-// a time.  The fused train tile at TILE = 16 runs k_raster_px2 instead: two
-// pixels per thread on sm_100's packed FP32 instructions, each warp covering
-// an 8x8 block, with results identical to k_raster's.
+// k_raster_warp runs every pass but the stored-state one: one warp per 8x8
+// block of a tile (TILE = 8, 16 or 32), two pixels per lane.  It is described
+// at the kernel.
 //
-// Forward: front-to-back compositing; the block leaves the tile when
-// __syncthreads_count (a block-wide ballot) finds every pixel saturated.  In
-// the fused train kernel each warp also records, per entry, whether any of
-// its pixels composited it (a ballot bit in shared memory): on dense scenes
-// only about a fifth of warp-entries composite anything.
-// Backward: each warp walks only the entries its bits mark, back to front
-// (without bits -- backward from saved state, or entries past the bit
-// capacity -- a warp-uniform test against the splat's conservative radius,
-// rad + 1 px, skips entries that cannot reach the warp's 8x4 pixels);
-// each pixel recovers the transmittance in front of a splat from the final
-// one (Tb = Ta / (1 - alpha)) -- or, in the stored-state variant, reads the
-// value the forward saved.  The ten gradient contributions of each pixel are
-// truncated to i32 fixed point (the reference's i32(clamp(v*16384, +-1e9)))
-// and summed exactly: a warp REDUX per slot, a shared-memory add per
-// (entry, slot) across the tile's warps, and one global atomic per (splat,
-// slot, tile).  Integer sums commute, so results are bit-identical in any
-// order -- the deterministic mode is the only mode.
+// k_raster_stored (forward + loss + backward that reads the transmittance the
+// forward saved, instead of recovering it from the final one): one CTA per
+// tile, one thread per pixel, each warp covering an 8x4 block.  Splat records
+// of the tile's sorted entries are staged in shared memory BATCH at a time;
+// the block leaves the tile's forward when __syncthreads_count (a block-wide
+// ballot) finds every pixel saturated.  Each warp records, per entry, whether
+// any of its pixels composited it (a ballot bit in shared memory), and the
+// backward walks the marked entries back to front (entries past the bit
+// capacity are all visited).
+//
+// The ten gradient contributions of each pixel are truncated to i32 fixed
+// point (the reference's i32(clamp(v*16384, +-1e9))) and summed exactly, with
+// a warp REDUX per slot and integer atomics.  Integer sums commute, so results
+// are bit-identical in any order -- the deterministic mode is the only mode.
 //
 // Control flow is warp-uniform (votes); per-lane work runs predicated, so
 // no divergent branch needs a reconvergence scaffold in the hot loops.
@@ -34,9 +28,13 @@
 // factors (gC, hence galpha, which is accumulated from the scaled gC):
 // scaling by a power of two is exact, so every truncated integer equals the
 // one the unfolded sequence produces.  The
-// +-1e9 clamp is skipped when a warp's scaled galpha is below 1e7: the
-// conic normaliser bounds every slot by 80 |galpha * 2^14| (slots 7-9 by
+// +-1e9 clamp is skipped when the scaled galpha is below 1e7: the conic
+// normaliser bounds every slot by 80 |galpha * 2^14| (slots 7-9 by
 // |gC * 2^14|), so the clamp cannot change a value then.
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
 #include "gs_common.cuh"
 #include "gs_kernels.h"
 
@@ -55,7 +53,7 @@ __device__ __forceinline__ float pairExponent(const float4& r0, float hC, float 
 __device__ __forceinline__ int32_t fix_scaled(float x) { return __float2int_rz(fminf(fmaxf(x, -1.0e9f), 1.0e9f)); }
 
 
-// Which of the tile's 8x4 warp blocks can the splat reach?  Bit w = warp w
+// Which of the tile's 8x4 warp blocks (k_raster_stored) can the splat reach?  Bit w = warp w
 // (block row w / (TILE/8), column w % (TILE/8)).  For each 4-row band, the
 // splat's pixels lie within |dx - kA dy| <= sqrt(p - q dmin^2) (cull
 // parameters (p, q, kA) from the projection; dmin = the band's smallest |dy|),
@@ -86,32 +84,31 @@ __device__ __forceinline__ uint32_t warp_block_mask(const float4 cq, float mx, f
 #define GS_RASTER16_MIN_BLOCKS 5  // resident 16x16-tile blocks per SM the register allocation must allow
 #endif
 // TILE x TILE pixels per CTA, one per thread; warps cover 8x4 blocks.
-template <int TILE, int BATCH, bool FWD, bool BWD, bool STORED>
-__global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOCKS : TILE == 8 ? 16 : 1) k_raster(RasterArgs a) {
+template <int TILE, int BATCH>
+__global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOCKS : TILE == 8 ? 16 : 1)
+    k_raster_stored(RasterArgs a) {
   constexpr int RT = TILE;
   constexpr int RTHREADS = TILE * TILE;
   constexpr int NW = RTHREADS / 32;  // warps
   constexpr int WPR = TILE / 8;      // 8-wide warp blocks per tile row
-  constexpr bool MASKS = FWD && BWD;
   static_assert(BATCH % 32 == 0, "batches hold whole ballot words");
   __shared__ RenderRec s_rec[BATCH];
   __shared__ uint32_t s_id[BATCH];
-  __shared__ int32_t s_acc[BWD ? BATCH * 10 : 1];
-  __shared__ uint32_t s_mask[MASKS ? NW * MASKW : 1];
-  __shared__ uint32_t s_live[FWD ? NW : 1][BATCH / 32];  // per warp: staged entries its block can reach
+  __shared__ int32_t s_acc[BATCH * 10];
+  __shared__ uint32_t s_mask[NW * MASKW];
+  __shared__ uint32_t s_live[NW][BATCH / 32];  // per warp: staged entries its block can reach
   __shared__ uint32_t s_item;
   __shared__ uint32_t s_redu[NW][5];
   __shared__ uint32_t s_endmax[NW];
-  __shared__ __align__(16) int32_t s_stage[BWD ? NW : 1][12];  // per warp: the 10 sums of one entry
+  __shared__ __align__(16) int32_t s_stage[NW][12];  // per warp: the 10 sums of one entry
 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int lx = (wid % WPR) * 8 + (lane & 7);
   const int ly = (wid / WPR) * 4 + (lane >> 3);
   const float E_CUT = a.eCut, A_MIN = a.aMin;
-  uint32_t* wmask = s_mask + (MASKS ? wid * MASKW : 0);
+  uint32_t* wmask = s_mask + wid * MASKW;
 
-  if (BWD)
-    for (int k = tid; k < BATCH * 10; k += RTHREADS) s_acc[k] = 0;
+  for (int k = tid; k < BATCH * 10; k += RTHREADS) s_acc[k] = 0;
 
   for (uint32_t iter = 0;; ++iter) {
     // ---- next work item (a global tile of the batch) ----
@@ -138,12 +135,10 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
     float T = 1.0f;
     float C0 = 0.0f, C1 = 0.0f, C2 = 0.0f;
     uint32_t cnt = e - s;  // one past the last processed entry (relative)
-    if (FWD) {
+    {
       bool done = !inside;
-      if (MASKS) {
-        for (int k = lane; k < MASKW; k += 32) wmask[k] = 0u;
-        __syncwarp();
-      }
+      for (int k = lane; k < MASKW; k += 32) wmask[k] = 0u;
+      __syncwarp();
       for (uint32_t base = s; base < e; base += BATCH) {
         if (__syncthreads_count(!done) == 0) break;
         const uint32_t nb = min((uint32_t)BATCH, e - base);
@@ -154,7 +149,7 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
           const uint32_t k = kb + tid;
           uint32_t m = 0;
           if (k < nb) {
-            const uint32_t id = a.ids[base + k];
+            const uint32_t id = a.ids[base + k] & a.idMask;
             s_id[k] = id;
             const RenderRec rec = recs[id];
             s_rec[k] = rec;
@@ -188,7 +183,7 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
                 const float araw = r1.y * gexp(-fminf(ee, 80.0f));
                 const float alpha = fminf(0.99f, araw);
                 const bool c2 = c1 && alpha >= A_MIN;
-                if (STORED && c2) a.tStore[(size_t)(base + jw + jj) * RTHREADS + tid] = T;
+                if (c2) a.tStore[(size_t)(base + jw + jj) * RTHREADS + tid] = T;
                 const float ta = T * alpha;
                 const float cb = rr.r2.x;
                 if (c2) {
@@ -198,13 +193,11 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
                   T = T * (1.0f - alpha);
                   if (T < 1e-4f) { done = true; cnt = rbase + jw + jj + 1; }
                 }
-                if (MASKS) bits |= (__ballot_sync(FULL, c2) != 0u ? 1u : 0u) << jj;
+                bits |= (__ballot_sync(FULL, c2) != 0u ? 1u : 0u) << jj;
               }
             }
-            if (MASKS) {
-              const uint32_t w = (rbase + jw) >> 5;
-              if (lane == 0 && w < MASKW) wmask[w] = bits;
-            }
+            const uint32_t w = (rbase + jw) >> 5;
+            if (lane == 0 && w < MASKW) wmask[w] = bits;
             if (__all_sync(FULL, done)) break;
           }
         }
@@ -214,18 +207,13 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
       C1 = C1 + T * c.bg[1];
       C2 = C2 + T * c.bg[2];
       if (inside) {
-        if (a.outImg) a.outImg[pix] = make_float4(C0, C1, C2, 1.0f - T);
-        if (a.finalT) a.finalT[pix] = T;
-        if (a.endIdx) a.endIdx[pix] = cnt;
+        a.outImg[pix] = make_float4(C0, C1, C2, 1.0f - T);
+        a.finalT[pix] = T;
+        a.endIdx[pix] = cnt;
       }
-    } else if (inside) {
-      const float4 o = a.outImg[pix];
-      C0 = o.x; C1 = o.y; C2 = o.z;
-      T = a.finalT[pix];
-      cnt = a.endIdx[pix];
     }
 
-    if (BWD) {
+    {
       // ---- loss (shaders.js:589-618) ----
       bool lossOk = false;
       float g16_0 = 0.0f, g16_1 = 0.0f, g16_2 = 0.0f;  // gC * 2^14
@@ -294,7 +282,7 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
         const uint32_t nb = hi - lo;
         __syncthreads();
         for (uint32_t k = tid; k < nb; k += RTHREADS) {
-          const uint32_t id = a.ids[s + lo + k];
+          const uint32_t id = a.ids[s + lo + k] & a.idMask;
           s_id[k] = id;
           s_rec[k] = recs[id];
         }
@@ -302,8 +290,7 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
         // this warp's entries in [lo, hi), back to front, one ballot word at a time
         for (int32_t w = (int32_t)((hi - 1) >> 5); w >= (int32_t)(lo >> 5); --w) {
           const uint32_t wb = (uint32_t)w << 5;
-          const bool haveBits = MASKS && (uint32_t)w < (uint32_t)MASKW;
-          uint32_t word = haveBits ? wmask[w] : FULL;
+          uint32_t word = (uint32_t)w < (uint32_t)MASKW ? wmask[w] : FULL;
           if (wb + 32u > hi) word &= FULL >> (wb + 32u - hi);
           if (wb < lo) word &= FULL << (lo - wb);
           while (word) {
@@ -327,7 +314,7 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
             const bool c2 = j < myEnd && ee <= E_CUT && alpha >= A_MIN;
             if (!__any_sync(FULL, c2)) continue;
             const float inv = rcp_unit(1.0f - alpha);  // 1 - alpha in [0.01, 1]: IEEE 1/x exactly
-            const float Tb = STORED ? (c2 ? a.tStore[(size_t)(s + j) * RTHREADS + tid] : 0.0f) : Ta * inv;
+            const float Tb = c2 ? a.tStore[(size_t)(s + j) * RTHREADS + tid] : 0.0f;
             const float aT = c2 ? alpha * Tb : 0.0f;
             const float g0 = __fmaf_rn(r1.z, Tb, -(S0 * inv));
             const float g1 = __fmaf_rn(r1.w, Tb, -(S1 * inv));
@@ -391,24 +378,15 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
   }
 }
 
-// Which 8x8 warp blocks of a 16x16 tile can the splat reach?  Bit w = warp w
-// (block row w / 2, column w % 2); the same band test as warp_block_mask on
-// 8-row bands.
-__device__ __forceinline__ uint32_t warp_block_mask8(const float4 cq, float mx, float my, int tx, int ty) {
-  if (!(cq.x < 3.0e38f)) return 0xFu;
-  uint32_t m = 0;
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    const float Y0 = ((float)(ty * 16 + 8 * b) + 0.5f) - my;
-    float xl, xr;
-    if (!bandIntervalMask(cq, Y0, Y0 + 7.0f, xl, xr)) continue;
-#pragma unroll
-    for (int wb = 0; wb < 2; ++wb) {
-      const float bx0 = ((float)(tx * 16 + 8 * wb) + 0.5f) - mx;
-      if (bx0 + 7.0f >= xl && bx0 <= xr) m |= 1u << (b * 2 + wb);
-    }
-  }
-  return m;
+// Can the splat (cull parameters cq, mean (mx, my)) reach the 8x8 pixel block
+// whose first pixel is (x0, y0)?  The same band test as warp_block_mask on an
+// 8-row band.
+__device__ __forceinline__ bool block_reach(const float4 cq, float mx, float my, int x0, int y0) {
+  if (!(cq.x < 3.0e38f)) return true;
+  const float Y0 = ((float)y0 + 0.5f) - my, X0 = ((float)x0 + 0.5f) - mx;
+  float xl, xr;
+  if (!bandIntervalMask(cq, Y0, Y0 + 7.0f, xl, xr)) return false;
+  return X0 + 7.0f >= xl && X0 <= xr;
 }
 
 // e = max(fma(fma(cA/2, dx, cB*dy), dx, ((cC/2)*dy)*dy), 0) for two pixels
@@ -426,442 +404,540 @@ __device__ __forceinline__ void cp_async_rec(RenderRec* dst, const RenderRec* sr
   cp_async16(&dst->r2, &src->r2);
 }
 
-#ifndef GS_RASTER_PX2_MIN_BLOCKS
-#define GS_RASTER_PX2_MIN_BLOCKS 8  // resident 128-thread blocks per SM the register allocation must allow
-#endif
-// Fused train tile (forward + loss + backward) on a 16x16 tile with two
-// pixels per thread: 128 threads, each warp covering an 8x8 block; lane l
-// holds pixels (l % 8, l / 8) and (l % 8, l / 8 + 4) of its block, which
-// share dx.  Every per-pixel operation runs on the pair with one packed
-// instruction (or twice, for comparisons, selects and conversions) and
-// performs the canonical sequence of k_raster on each pixel; the per-entry
-// work (record loads, votes, the ten warp reductions and the shared-memory
-// adds) is shared by 64 pixels instead of 32.  Results are bit-identical to
-// k_raster<16, BATCH, true, true, false>: the same entries reach every pixel
-// (an 8x8 block skips an entry only when neither of its 8x4 halves can use
-// it), and integer sums do not depend on how pixels are grouped.
-//
-// Staging: each batch of BATCH entries is copied from global to shared
-// memory with cp.async (16-byte copies, no register round trip); the entry
-// ids of the next batch are loaded into registers while the current one is
-// processed, so a batch's staging waits for one gather, not for the id load
-// and then the gather.  Each thread copies its own entries (k = tid,
-// tid + 128) and, in the forward, computes their warp-block masks from its
-// own completed copies before the batch's barrier.  (Double-buffering the
-// records as well -- the next batch copied while the current one is
-// processed -- needs twice the record storage, which at 256 entries drops
-// the block from 8 to 5 resident per SM; measured, it did not pay.)
-template <int BATCH>
-__global__ void __launch_bounds__(128, GS_RASTER_PX2_MIN_BLOCKS) k_raster_px2(RasterArgs a) {
-  constexpr int NT = 128, NW = 4;
-  constexpr int PER = BATCH >= NT ? BATCH / NT : 1;  // entries a thread stages per batch
-  static_assert(BATCH % 32 == 0, "batches hold whole ballot words");
-  static_assert(BATCH <= 2 * NT, "two staged entries per thread");
-  __shared__ RenderRec s_rec[BATCH];
-  // the forward's cull parameters and the backward's per-entry sums share storage
-  constexpr int ACC_WORDS = BATCH * 10, CULL_WORDS = BATCH * 4;
-  __shared__ __align__(16) int32_t s_accu[ACC_WORDS > CULL_WORDS ? ACC_WORDS : CULL_WORDS];
-  int32_t* s_acc = s_accu;
-  float4* s_cull = reinterpret_cast<float4*>(s_accu);
-  __shared__ uint32_t s_id[BATCH];
-  __shared__ uint32_t s_mask[NW * MASKW];
-  __shared__ uint32_t s_live[NW][BATCH / 32];
-  __shared__ uint32_t s_item;
-  __shared__ uint32_t s_redu[NW][5];
-  __shared__ uint32_t s_endmax[NW];
-  __shared__ __align__(16) int32_t s_stage[NW][12];
+// Shared memory by 32-bit address: the hot loops step such an address in one
+// register.  (Indexing the arrays instead had the compiler form the address
+// anew for every entry.)
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  uint32_t r;  // opaque, so that it stays in a register
+  asm volatile("mov.u32 %0, %1;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+  return r;
+}
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds1(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts4(uint32_t a, int x, int y, int z, int w) {
+  asm volatile("st.shared.v4.s32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void sts2(uint32_t a, int x, int y) {
+  asm volatile("st.shared.v2.s32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+// *p += v unless v is 0, without a branch
+__device__ __forceinline__ void red_nz(int32_t* p, int32_t v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.s32 q, %1, 0;\n @q red.global.add.s32 [%0], %1;\n}" ::"l"(p), "r"(v)
+               : "memory");
+}
 
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int lx = (wid & 1) * 8 + (lane & 7);
-  const int ly = (wid >> 1) * 8 + (lane >> 3);  // pixel a; pixel b is 4 rows below
-  const float E_CUT = a.eCut, A_MIN = a.aMin;
-  uint32_t* wmask = s_mask + wid * MASKW;
+struct StagedRec {
+  RenderRec rec;
+  uint32_t id;   // splat
+  uint32_t raw;  // place in its chunk of list entries
+  uint32_t pad[2];
+};
+// The rasteriser: one warp per 8x8 pixel block of a tile, with no barrier
+// between warps.  Lane l holds pixels (l % 8, l / 8) and (l % 8, l / 8 + 4),
+// which share dx; every per-pixel operation runs on the pair as one packed
+// instruction (or twice, for comparisons, selects and conversions).
+//
+// Forward: the tile's list is read 32 entries at a time.  An entry whose
+// block bit is clear cannot reach the block (k_expand computed the bits; with
+// MASKED off the warp tests the cull parameters itself); the records of the
+// others are copied to shared memory with cp.async, compacted, one chunk
+// ahead of the one being composited.
+// Backward (BWD): walks the composited entries back to front.  The forward
+// left their ids and, per pixel, the exponential G (0 where the pixel did not
+// composite the entry) in the warp's slice of a cache in global memory, so the
+// backward neither evaluates the exponential again nor tests the cutoffs.
+// Entries past the slice (cacheCap of them fit) are recomputed from the list.
+// The ten integer sums of an entry go from the warp straight to gradP.
+//
+// What bounds it: instruction issue (70% active), with the conversions to
+// integers (F2I: 8 cycles a warp) at 55% of their pipe and FMA at 57%.  Measured
+// on 1M splats, two 1080p views: 2.06 ms, 1.62 G warp instructions; the block
+// per tile of four warps it replaced, which met at a barrier every batch and
+// recomputed G: 2.49 ms, 2.08 G.  The cache moves 3.1 GB through DRAM in that
+// time (1.5 TB/s), loads two entries ahead; without it the pass is 9% slower.
+//
+// MINB: resident blocks per SM that the registers allow.  7 (72 registers) is
+// best while there is enough work to keep every SM full, and 5 (80 registers)
+// when fewer blocks run (raster_grid).
+template <int TILE, bool MASKED, bool BWD, int MINB>
+__global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs a) {
+  constexpr int SUB = (TILE / 8) * (TILE / 8);  // 8x8 blocks per tile
+  constexpr int SPR = TILE / 8;                 // of them in one row
+  static_assert(!MASKED || TILE <= 16, "entry values carry at most four block bits");
+  __shared__ StagedRec s_rec[RW_WARPS][2][32];
+  __shared__ __align__(128) int32_t s_stage[BWD ? RW_WARPS : 1][2][16];
+  __shared__ uint32_t s_stat[3];
+  __shared__ int32_t s_cam[MAX_VIEWS][2];
+
+  const int wid = threadIdx.x >> 5;
+  int lane;  // opaque, so that it stays in a register instead of being read again per entry
+  asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+  // alpha = min(0.99, w G) is tested as w G, which is the same for cutoffs up
+  // to 0.99 (a larger one accepts nothing)
+  const float E_CUT = a.eCut, A_MIN = a.aMin <= 0.99f ? a.aMin : __int_as_float(0x7F800000);
+  const uint32_t ltm = (1u << lane) - 1u;
+  if (BWD) {
+    if (threadIdx.x < 3) s_stat[threadIdx.x] = 0u;
+    if (threadIdx.x < 2 * MAX_VIEWS) (&s_cam[0][0])[threadIdx.x] = 0;
+    if (threadIdx.x < RW_WARPS * 2) s_stage[threadIdx.x >> 1][threadIdx.x & 1][10] = 0;  // word 10 of each row
+    __syncthreads();
+  }
+  const uint32_t warp = blockIdx.x * RW_WARPS + (uint32_t)wid;
+  const uint32_t items = a.totalTiles * (uint32_t)SUB;
+  // this warp's slice of the exponential cache: slots 2 to cacheCap + 1 keep
+  // entries.  The slot after the last kept one takes the stores of entries
+  // that are not kept, which for a full slice is slot 0 of the next one;
+  // slots 0 and 1 are only ever loaded ahead of use, and never used.
+  const uint32_t slice = BWD ? (warp % a.cacheWarps) * (a.cacheCap + 2u) : 0u;
+  float2* const gFirst = BWD ? a.cacheG + ((size_t)(slice + 2u) * 32 + lane) : nullptr;
+  uint32_t* const cacheId = BWD ? a.cacheId + slice : nullptr;
 
   for (uint32_t iter = 0;; ++iter) {
-    if (tid == 0) s_item = a.workCounter ? atomicAdd(a.workCounter, 1u) : (iter == 0 ? blockIdx.x : 0xFFFFFFFFu);
-    __syncthreads();
-    const uint32_t item = s_item;
-    __syncthreads();
-    if (item >= a.totalTiles) break;
-    const uint32_t gt = a.workOrder ? a.workOrder[item] : item;
+    uint32_t item = iter == 0 ? warp : 0xFFFFFFFFu;
+    if (a.workCounter) {
+      if (lane == 0) item = atomicAdd(a.workCounter, 1u);
+      item = __shfl_sync(FULL, item, 0);
+    }
+    if (item >= items) break;
+    const uint32_t ti = item / SUB, sub = item % SUB;
+    const uint32_t gt = a.workOrder ? a.workOrder[ti] : ti;
     int v = 0;
     while (v + 1 < a.V && a.cams[v + 1].tileBase <= gt) ++v;
     const DevCam& c = a.cams[v];
     const uint32_t t = gt - c.tileBase;
-    const int tx = (int)(t % (uint32_t)c.tilesX), ty = (int)(t / (uint32_t)c.tilesX);
-    const int x = tx * 16 + lx, ya = ty * 16 + ly, yb = ya + 4;
+    const int x = (int)(t % (uint32_t)c.tilesX) * TILE + (int)(sub % SPR) * 8 + (lane & 7);
+    const int ya = (int)(t / (uint32_t)c.tilesX) * TILE + (int)(sub / SPR) * 8 + (lane >> 3), yb = ya + 4;
     const bool inA = x < c.W && ya < c.H, inB = x < c.W && yb < c.H;
+    if (!__any_sync(FULL, inA)) continue;  // the block lies outside the image
     const float px = (float)x + 0.5f;
     const float2 py = make_float2((float)ya + 0.5f, (float)yb + 0.5f);
     const uint2 rg = a.ranges[gt];
     const uint32_t s = rg.x, e = rg.y;
-    const size_t pixA = (size_t)c.pixBase + (size_t)ya * c.W + x;
-    const size_t pixB = pixA + (size_t)4 * c.W;
     const RenderRec* recs = a.recs + (size_t)v * a.n;
-    const float4* cullRecs = a.cullRecs + (size_t)v * a.n;
 
-    // ---- forward ----
-    float2 T = bc2(1.0f);
-    float2 C0 = bc2(0.0f), C1 = bc2(0.0f), C2 = bc2(0.0f);
-    uint32_t cntA = e - s, cntB = e - s;
-    bool doneA = !inA, doneB = !inB;
-    for (int k = lane; k < MASKW; k += 32) wmask[k] = 0u;
-    __syncwarp();
-    // ids of entries [from, to) that this thread stages (k = tid, tid + 128)
-    uint32_t pf[PER];
-    auto load_ids = [&](uint32_t from, uint32_t to) {
-#pragma unroll
-      for (int u = 0; u < PER; ++u) {
-        const uint32_t k = (uint32_t)(u * NT + tid);
-        pf[u] = k < (uint32_t)BATCH && from + k < to ? a.ids[from + k] : 0u;
-      }
-    };
-    load_ids(s, e);
-    for (uint32_t base = s; base < e; base += BATCH) {
-      // every warp has finished the previous batch: its buffers may be overwritten
-      if (__syncthreads_count(!(doneA && doneB)) == 0) break;
-      const uint32_t nb = min((uint32_t)BATCH, e - base);
-#pragma unroll
-      for (int u = 0; u < PER; ++u) {
-        const uint32_t k = (uint32_t)(u * NT + tid);
-        if (k < nb) {
-          cp_async_rec(&s_rec[k], recs + pf[u]);
-          cp_async16(&s_cull[k], cullRecs + pf[u]);
+    // Stage the chunk of entry values `val` (lane l: list entry base + l) into
+    // buffer b: the live entries' records, compacted.  Returns their bits.
+    auto stage = [&](uint32_t val, bool have, int b) {
+      bool live = have;
+      uint32_t id = val;
+      if (MASKED) {
+        id = val & ID_MASK;
+        live = have && ((val >> (ID_BITS + sub)) & 1u);
+      } else if (TILE > 8) {
+        if (have) {
+          const float4 cq = a.cullRecs[(size_t)v * a.n + id];
+          const float2 m = *reinterpret_cast<const float2*>(&recs[id].r0);
+          live = block_reach(cq, m.x, m.y, x - (lane & 7), ya - (lane >> 3));
         }
+      }
+      const uint32_t bits = __ballot_sync(FULL, live);
+      if (live) {
+        const uint32_t pos = (uint32_t)__popc(bits & ltm);
+        StagedRec* d = &s_rec[wid][b][pos];
+        cp_async_rec(&d->rec, recs + id);
+        d->id = id;
+        d->raw = (uint32_t)lane;
       }
       cp_async_commit();
-      load_ids(base + BATCH, e);  // the next batch's ids load while this one is processed
-      cp_async_wait<0>();         // this thread's copies have landed
-#pragma unroll
-      for (int u = 0; u < (BATCH + NT - 1) / NT; ++u) {
-        const uint32_t kb = (uint32_t)(u * NT);
-        const uint32_t k = kb + tid;
-        uint32_t m = 0;
-        if (k < nb) m = warp_block_mask8(s_cull[k], s_rec[k].r0.x, s_rec[k].r0.y, tx, ty);
-        const uint32_t word = (kb >> 5) + (uint32_t)wid;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-          const uint32_t bw = __ballot_sync(FULL, (m >> w) & 1u);
-          if (lane == 0 && word < (uint32_t)(BATCH / 32)) s_live[w][word] = bw;
+      return bits;
+    };
+
+    // ---- forward ----
+    // A pixel is done once its transmittance is below 1e-4; pixels outside the
+    // image start at 0, so they never composite.
+    float2 T = make_float2(inA ? 1.0f : 0.0f, inB ? 1.0f : 0.0f);
+    float2 C0 = bc2(0.0f), C1 = bc2(0.0f), C2 = bc2(0.0f);
+    uint32_t cntA = 0u, cntB = 0u;  // end index of a pixel that is done, 0 before
+    float2* gp = gFirst;            // next cache slot
+    uint32_t uncached = e;          // first list entry (at a chunk start) past the cache
+    uint32_t seenEnd = s;           // one past the last chunk processed
+    {
+      auto load = [&](uint32_t base) { return base + lane < e ? a.ids[base + lane] : 0u; };
+      int b = 0;
+      uint32_t bits = stage(load(s), s + lane < e, 0);
+      uint32_t nextVal = s + 32 < e ? load(s + 32) : 0u;
+      for (uint32_t base = s; base < e; base += 32) {
+        uint32_t nextBits = 0;
+        if (base + 32 < e) {
+          nextBits = stage(nextVal, base + 32 + lane < e, b ^ 1);
+          nextVal = base + 64 < e ? load(base + 64) : 0u;
+          cp_async_wait<1>();
+        } else {
+          cp_async_wait<0>();
         }
-      }
-      __syncthreads();
-      if (!__all_sync(FULL, doneA && doneB)) {
-        const uint32_t rbase = base - s;
-        for (uint32_t jw = 0; jw < nb; jw += 32) {
-          uint32_t live = s_live[wid][jw >> 5];
-          uint32_t bits = 0;
-          while (live) {
-            const uint32_t jj = (uint32_t)__ffs(live) - 1u;
-            live &= live - 1u;
-            const RenderRec& rr = s_rec[jw + jj];
-            const float4 r0 = rr.r0;
-            const float4 r1 = rr.r1;
-            const float dx = px - r0.x;
-            const float2 dy = __fadd2_rn(py, bc2(-r0.y));
-            float2 Bdy;
-            const float2 ee = pairExponent2(r0, r1.x, dx, dy, Bdy);
-            const bool c1a = !doneA && ee.x <= E_CUT, c1b = !doneB && ee.y <= E_CUT;
-            if (__any_sync(FULL, c1a || c1b)) {
-              const float2 G = gexp2(make_float2(-fminf(ee.x, 80.0f), -fminf(ee.y, 80.0f)));
-              const float2 araw = __fmul2_rn(bc2(r1.y), G);
-              const float2 alpha = make_float2(fminf(0.99f, araw.x), fminf(0.99f, araw.y));
-              const bool c2a = c1a && alpha.x >= A_MIN, c2b = c1b && alpha.y >= A_MIN;
-              // a pixel that does not composite sees alpha 0: C and T stay exactly as they are
-              const float2 am = make_float2(c2a ? alpha.x : 0.0f, c2b ? alpha.y : 0.0f);
-              const float2 ta = __fmul2_rn(T, am);
-              C0 = __ffma2_rn(ta, bc2(r1.z), C0);
-              C1 = __ffma2_rn(ta, bc2(r1.w), C1);
-              C2 = __ffma2_rn(ta, bc2(rr.r2.x), C2);
-              T = __fmul2_rn(T, __fadd2_rn(bc2(1.0f), make_float2(-am.x, -am.y)));
-              if (c2a && T.x < 1e-4f) { doneA = true; cntA = rbase + jw + jj + 1; }
-              if (c2b && T.y < 1e-4f) { doneB = true; cntB = rbase + jw + jj + 1; }
-              bits |= (__ballot_sync(FULL, c2a || c2b) != 0u ? 1u : 0u) << jj;
+        __syncwarp();
+        const uint32_t n = (uint32_t)__popc(bits);
+        if (BWD && uncached == e && (uint32_t)((gp - gFirst) >> 5) + n > a.cacheCap) uncached = base;
+        const uint32_t step = BWD && uncached == e ? 32u : 0u;
+        uint32_t hit = 0;
+        uint32_t kA = 0, kB = 0;  // last entry of the chunk that each pixel composited
+        const StagedRec* sr = s_rec[wid][b];
+        for (uint32_t k = 0; k < n; ++k, ++sr) {
+          const float4 r0 = sr->rec.r0;
+          const float4 r1 = sr->rec.r1;
+          const float dx = px - r0.x;
+          const float2 dy = __fadd2_rn(py, bc2(-r0.y));
+          float2 Bdy;
+          const float2 ee = pairExponent2(r0, r1.x, dx, dy, Bdy);
+          // beyond the cutoff (at most 80) G may be anything: it is masked below
+          const float2 G = gexp2(make_float2(-ee.x, -ee.y));
+          const float2 araw = __fmul2_rn(bc2(r1.y), G);
+          const bool c2a = T.x >= 1e-4f && ee.x <= E_CUT && araw.x >= A_MIN;
+          const bool c2b = T.y >= 1e-4f && ee.y <= E_CUT && araw.y >= A_MIN;
+          // a pixel that does not composite sees alpha 0: C and T stay exactly as they are
+          const float2 Gm = make_float2(c2a ? G.x : 0.0f, c2b ? G.y : 0.0f);
+          const float2 aw = __fmul2_rn(bc2(r1.y), Gm);
+          const float2 am = make_float2(fminf(0.99f, aw.x), fminf(0.99f, aw.y));
+          const float2 ta = __fmul2_rn(T, am);
+          C0 = __ffma2_rn(ta, bc2(r1.z), C0);
+          C1 = __ffma2_rn(ta, bc2(r1.w), C1);
+          C2 = __ffma2_rn(ta, bc2(sr->rec.r2.x), C2);
+          T = __fmul2_rn(T, __fadd2_rn(bc2(1.0f), make_float2(-am.x, -am.y)));
+          kA = c2a ? k : kA;
+          kB = c2b ? k : kB;
+          if (BWD) {
+            __stcg(gp, Gm);
+            hit >>= 1;
+            if (__any_sync(FULL, c2a || c2b)) {
+              hit |= 0x80000000u;
+              gp += step;
             }
           }
-          const uint32_t w = (rbase + jw) >> 5;
-          if (lane == 0 && w < MASKW) wmask[w] = bits;
-          if (__all_sync(FULL, doneA && doneB)) break;
         }
+        hit = n ? hit >> (32u - n) : 0u;  // bit k: entry k
+        if (step && ((hit >> lane) & 1u))
+          __stcg(cacheId + ((uint32_t)((gp - gFirst) >> 5) - (uint32_t)__popc(hit & ~ltm)), s_rec[wid][b][lane].id);
+        if (T.x < 1e-4f && cntA == 0u) cntA = base - s + s_rec[wid][b][kA].raw + 1u;
+        if (T.y < 1e-4f && cntB == 0u) cntB = base - s + s_rec[wid][b][kB].raw + 1u;
+        seenEnd = base + 32;
+        if (__all_sync(FULL, T.x < 1e-4f && T.y < 1e-4f)) break;
+        __syncwarp();  // every lane is done with buffer b: the next chunk but one may overwrite it
+        bits = nextBits;
+        b ^= 1;
       }
+      cp_async_wait<0>();
+      __syncwarp();
+      if (cntA == 0u) cntA = e - s;
+      if (cntB == 0u) cntB = e - s;
     }
     C0 = __fadd2_rn(C0, __fmul2_rn(T, bc2(c.bg[0])));
     C1 = __fadd2_rn(C1, __fmul2_rn(T, bc2(c.bg[1])));
     C2 = __fadd2_rn(C2, __fmul2_rn(T, bc2(c.bg[2])));
-    if (inA) {
-      if (a.outImg) a.outImg[pixA] = make_float4(C0.x, C1.x, C2.x, 1.0f - T.x);
-      if (a.finalT) a.finalT[pixA] = T.x;
-      if (a.endIdx) a.endIdx[pixA] = cntA;
+    {
+      const size_t pixA = (size_t)c.pixBase + (size_t)ya * c.W + x;
+      const size_t pixB = pixA + (size_t)4 * c.W;
+      if (inA) {
+        a.outImg[pixA] = make_float4(C0.x, C1.x, C2.x, 1.0f - T.x);
+        a.finalT[pixA] = T.x;
+        a.endIdx[pixA] = cntA;
+      }
+      if (inB) {
+        a.outImg[pixB] = make_float4(C0.y, C1.y, C2.y, 1.0f - T.y);
+        a.finalT[pixB] = T.y;
+        a.endIdx[pixB] = cntB;
+      }
     }
-    if (inB) {
-      if (a.outImg) a.outImg[pixB] = make_float4(C0.y, C1.y, C2.y, 1.0f - T.y);
-      if (a.finalT) a.finalT[pixB] = T.y;
-      if (a.endIdx) a.endIdx[pixB] = cntB;
-    }
+    if (!BWD) continue;
 
     // ---- loss (shaders.js:589-618), per pixel ----
     float2 g16_0 = bc2(0.0f), g16_1 = bc2(0.0f), g16_2 = bc2(0.0f);
-    uint32_t st0 = 0, st1 = 0, st2 = 0, cg6 = 0, cg7 = 0;
-    uint32_t myEndA = 0, myEndB = 0;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool in = h ? inB : inA;
-      if (!in) continue;
-      const int yy = h ? yb : ya;
-      const uint32_t pi = (uint32_t)(yy * c.W + x);
-      const uint32_t packed = a.targets[(size_t)c.offset + pi];
-      if ((packed >> 24) == 0u) continue;
-      const float Cx = h ? C0.y : C0.x, Cy = h ? C1.y : C1.x, Cz = h ? C2.y : C2.x;
-      const float t0 = (float)(packed & 0xFFu) / 255.0f;
-      const float t1 = (float)((packed >> 8) & 0xFFu) / 255.0f;
-      const float t2 = (float)((packed >> 16) & 0xFFu) / 255.0f;
-      st2 += 1u;
-      const float gain = c.gain;
-      const float er0 = (gain * Cx + c.bias) - t0;
-      const float er1 = (gain * Cy + c.bias) - t1;
-      const float er2 = (gain * Cz + c.bias) - t2;
-      st0 += u32sat((er0 * er0 + er1 * er1 + er2 * er2) * 16.0f + dither(pi));
-      const float D2 = 9.0000000000000003e-04f;  // f32(0.03 * 0.03), a WGSL const-expression
-      const float rt0 = sqrtf(er0 * er0 + D2), rt1 = sqrtf(er1 * er1 + D2), rt2 = sqrtf(er2 * er2 + D2);
-      const float eg0 = er0 / rt0, eg1 = er1 / rt1, eg2 = er2 / rt2;
-      const float q0 = gain * eg0, q1 = gain * eg1, q2 = gain * eg2;
-      const float lossv = (rt0 + rt1 + rt2) - 8.9999999999999997e-02f;  // f32(3 * 0.03)
-      st1 += u32sat(lossv * 32768.0f);
-      cg6 += (uint32_t)fixq((eg0 * Cx + eg1 * Cy + eg2 * Cz) * gain, FIXCAM);
-      cg7 += (uint32_t)fixq(eg0 + eg1 + eg2, FIXCAM);
-      if (h) {
-        g16_0.y = q0 * FIXED; g16_1.y = q1 * FIXED; g16_2.y = q2 * FIXED;
-        myEndB = cntB;
-      } else {
-        g16_0.x = q0 * FIXED; g16_1.x = q1 * FIXED; g16_2.x = q2 * FIXED;
-        myEndA = cntA;
-      }
-    }
-    // slots 7-9 stay within +-1e9 without clamping when |gC * 2^14| < 9e8
-    const bool pixFast = fabsf(g16_0.x) < 9.0e8f && fabsf(g16_1.x) < 9.0e8f && fabsf(g16_2.x) < 9.0e8f &&
-                         fabsf(g16_0.y) < 9.0e8f && fabsf(g16_1.y) < 9.0e8f && fabsf(g16_2.y) < 9.0e8f;
+    bool okA = false, okB = false;  // pixels with a valid target
     {
+      uint32_t st0 = 0, st1 = 0, st2 = 0, cg6 = 0, cg7 = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const bool in = h ? inB : inA;
+        if (!in) continue;
+        const int yy = h ? yb : ya;
+        const uint32_t pi = (uint32_t)(yy * c.W + x);
+        const uint32_t packed = a.targets[(size_t)c.offset + pi];
+        if ((packed >> 24) == 0u) continue;
+        const float Cx = h ? C0.y : C0.x, Cy = h ? C1.y : C1.x, Cz = h ? C2.y : C2.x;
+        const float t0 = (float)(packed & 0xFFu) / 255.0f;
+        const float t1 = (float)((packed >> 8) & 0xFFu) / 255.0f;
+        const float t2 = (float)((packed >> 16) & 0xFFu) / 255.0f;
+        st2 += 1u;
+        const float gain = c.gain;
+        const float er0 = (gain * Cx + c.bias) - t0;
+        const float er1 = (gain * Cy + c.bias) - t1;
+        const float er2 = (gain * Cz + c.bias) - t2;
+        st0 += u32sat((er0 * er0 + er1 * er1 + er2 * er2) * 16.0f + dither(pi));
+        const float D2 = 9.0000000000000003e-04f;  // f32(0.03 * 0.03), a WGSL const-expression
+        const float rt0 = sqrtf(er0 * er0 + D2), rt1 = sqrtf(er1 * er1 + D2), rt2 = sqrtf(er2 * er2 + D2);
+        const float eg0 = er0 / rt0, eg1 = er1 / rt1, eg2 = er2 / rt2;
+        const float q0 = gain * eg0, q1 = gain * eg1, q2 = gain * eg2;
+        const float lossv = (rt0 + rt1 + rt2) - 8.9999999999999997e-02f;  // f32(3 * 0.03)
+        st1 += u32sat(lossv * 32768.0f);
+        cg6 += (uint32_t)fixq((eg0 * Cx + eg1 * Cy + eg2 * Cz) * gain, FIXCAM);
+        cg7 += (uint32_t)fixq(eg0 + eg1 + eg2, FIXCAM);
+        if (h) {
+          g16_0.y = q0 * FIXED; g16_1.y = q1 * FIXED; g16_2.y = q2 * FIXED;
+          okB = true;
+        } else {
+          g16_0.x = q0 * FIXED; g16_1.x = q1 * FIXED; g16_2.x = q2 * FIXED;
+          okA = true;
+        }
+      }
+      // wrapping sums of the per-pixel stats, kept per block until the kernel's end
       const uint32_t r0 = __reduce_add_sync(FULL, st0);
       const uint32_t r1 = __reduce_add_sync(FULL, st1);
       const uint32_t r2 = __reduce_add_sync(FULL, st2);
       const uint32_t r3 = __reduce_add_sync(FULL, cg6);
       const uint32_t r4 = __reduce_add_sync(FULL, cg7);
-      const uint32_t mx = __reduce_max_sync(FULL, max(myEndA, myEndB));
       if (lane == 0) {
-        s_redu[wid][0] = r0; s_redu[wid][1] = r1; s_redu[wid][2] = r2;
-        s_redu[wid][3] = r3; s_redu[wid][4] = r4;
-        s_endmax[wid] = mx;
+        atomicAdd(&s_stat[0], r0);
+        atomicAdd(&s_stat[1], r1);
+        atomicAdd(&s_stat[2], r2);
+        atomicAdd(&s_cam[v][0], (int32_t)r3);
+        atomicAdd(&s_cam[v][1], (int32_t)r4);
       }
     }
-    __syncthreads();
-    if (tid < 5) {
-      uint32_t sum = 0;
-      for (int w = 0; w < NW; ++w) sum += s_redu[w][tid];
-      if (sum) {
-        if (tid < 3) atomicAdd(&a.stats[tid], sum);
-        else atomicAdd(&a.gradCam[c.camIdx * 8u + 3u + (uint32_t)tid], (int32_t)sum);
-      }
-    }
-    uint32_t endMax = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) endMax = max(endMax, s_endmax[w]);
-    // the forward's cull parameters shared storage with the per-entry sums:
-    // every reader of them has passed the barrier above
-    for (int k = tid; k < BATCH * 10; k += NT) s_acc[k] = 0;
+    if (!__any_sync(FULL, okA || okB)) continue;
+    // Clamping (see fix_scaled) changes nothing while every value stays within
+    // +-1e9: slots 0-6 within 80 |galpha * 2^14|, slots 7-9 within |gC * 2^14|.
+    // galpha is at most the pixel's sum of |gC| times the largest colour of
+    // the splats from the back to here (a blend of them in front of or behind
+    // the splat, times a transmittance of at most 1); 2.5 leaves room for the
+    // rounding.  Both maxima are taken on the float's bits, so infinities and
+    // NaN count as larger than every number.
+    const float gMax = __uint_as_float(__reduce_max_sync(
+        FULL, max(__float_as_uint(fabsf(g16_0.x) + fabsf(g16_1.x) + fabsf(g16_2.x)),
+                  __float_as_uint(fabsf(g16_0.y) + fabsf(g16_1.y) + fabsf(g16_2.y)))));
+    uint32_t cMax = __float_as_uint(fmaxf(fabsf(c.bg[0]), fmaxf(fabsf(c.bg[1]), fabsf(c.bg[2]))));
+    bool fast = false;
+    auto widen = [&](const StagedRec* sr, uint32_t n) {  // the chunk's colours join cMax
+      uint32_t m = 0;
+      if ((uint32_t)lane < n)
+        m = max(__float_as_uint(fabsf(sr[lane].rec.r1.z)),
+                max(__float_as_uint(fabsf(sr[lane].rec.r1.w)), __float_as_uint(fabsf(sr[lane].rec.r2.x))));
+      cMax = max(cMax, __reduce_max_sync(FULL, m));
+      fast = gMax < 9.0e8f && gMax * 2.5f * __uint_as_float(cMax) < 1.0e7f;
+    };
 
     // ---- backward (shaders.js:632-700) ----
     float2 S0 = __fmul2_rn(bc2(c.bg[0]), T), S1 = __fmul2_rn(bc2(c.bg[1]), T), S2 = __fmul2_rn(bc2(c.bg[2]), T);
     float2 Ta = T;
-    int32_t* gradP = a.gradP + (size_t)v * a.n * GP_STRIDE;
-    // batches run back to front: [lo, hi) with hi = endMax, then hi = lo;
-    // each batch's ids are loaded while the batch before it is processed
-    auto lo_of = [](uint32_t hi) { return hi > (uint32_t)BATCH ? hi - (uint32_t)BATCH : 0u; };
-    if (endMax > 0) load_ids(s + lo_of(endMax), s + endMax);
-    for (uint32_t hi = endMax; hi > 0;) {
-      const uint32_t lo = lo_of(hi);
-      const uint32_t nb = hi - lo;
-      __syncthreads();  // the previous batch's processing and flush are over
+    int32_t* gradP = a.gradP + (size_t)v * a.n * GP_STRIDE + lane;
+    asm volatile("mov.u64 %0, %1;" : "=l"(gradP) : "l"(gradP));  // opaque: not formed anew per entry
+    uint32_t row = smem_addr(s_stage[wid][0]);  // the staging row in use; the other is 64 bytes away
+    uint32_t slotOff;                            // this lane's word of a row
+    asm volatile("mov.u32 %0, %1;" : "=r"(slotOff) : "r"((lane < 10 ? lane : 10) * 4));
+    // One composited entry at shared address sr, G the pixels' exponentials (0
+    // where a pixel does not composite it).  FAST: every product is finite and
+    // within +-1e9, so a pixel with G = 0 or without a target (gC = 0)
+    // contributes zeros without being masked.
+    auto backward = [&](uint32_t sr, float2 G, auto FAST) {
+      const float4 r0 = lds4(sr);
+      const float4 r1 = lds4(sr + 16);
+      const float4 r2 = lds4(sr + 32);
+      const float dx = px - r0.x, dx2 = dx + dx;
+      const float2 dy = __fadd2_rn(py, bc2(-r0.y)), dy2 = __fadd2_rn(dy, dy);
+      const float2 Bdy = __fmul2_rn(bc2(r0.w), dy);
+      const float2 araw = __fmul2_rn(bc2(r1.y), G);
+      const float2 alpha = make_float2(fminf(0.99f, araw.x), fminf(0.99f, araw.y));
+      const float2 inv = rcp_unit2(__fadd2_rn(bc2(1.0f), make_float2(-alpha.x, -alpha.y)));
+      // a pixel that does not composite has alpha 0: inv is 1, and Ta and S stay exactly as they are
+      const float2 Tb = __fmul2_rn(Ta, inv);
+      const float2 aT = __fmul2_rn(alpha, Tb);
+      const float2 g0 = __ffma2_rn(bc2(r1.z), Tb, __fmul2_rn(make_float2(-S0.x, -S0.y), inv));
+      const float2 g1 = __ffma2_rn(bc2(r1.w), Tb, __fmul2_rn(make_float2(-S1.x, -S1.y), inv));
+      const float2 g2 = __ffma2_rn(bc2(r2.x), Tb, __fmul2_rn(make_float2(-S2.x, -S2.y), inv));
+      // galpha * 2^14, accumulated from gC * 2^14
+      const float2 gal16r = __ffma2_rn(g16_2, g2, __ffma2_rn(g16_1, g1, __fmul2_rn(g16_0, g0)));
+      const bool useA = decltype(FAST)::value || (okA && G.x > 0.0f), useB = decltype(FAST)::value || (okB && G.y > 0.0f);
+      const float2 gal16 = make_float2(useA && !(araw.x > 0.99f) ? gal16r.x : 0.0f,
+                                       useB && !(araw.y > 0.99f) ? gal16r.y : 0.0f);
+      const float2 ga16 = __fmul2_rn(gal16, araw);
+      const float2 gq16 = __fmul2_rn(ga16, bc2(r2.z));
+      const float2 gqx16 = __fmul2_rn(gq16, bc2(dx));
+      // the conic's halves times doubled offsets: doubling commutes with rounding
+      float2 xs[10];
+      xs[0] = __fmul2_rn(ga16, __ffma2_rn(bc2(r0.z), bc2(dx2), Bdy));
+      xs[1] = __fmul2_rn(ga16, __ffma2_rn(bc2(r0.w), bc2(dx), __fmul2_rn(bc2(r1.x), dy2)));
+      xs[2] = __fmul2_rn(gqx16, bc2(dx));
+      xs[3] = __fmul2_rn(gqx16, dy2);
+      xs[4] = __fmul2_rn(__fmul2_rn(gq16, dy), dy);
+      xs[5] = __fmul2_rn(__fmul2_rn(gal16, bc2(r2.y)), G);
+      xs[6] = __fmul2_rn(ga16, bc2(r2.w));
+      xs[7] = __fmul2_rn(g16_0, aT);
+      xs[8] = __fmul2_rn(g16_1, aT);
+      xs[9] = __fmul2_rn(g16_2, aT);
+      if (!decltype(FAST)::value &&
+          !__all_sync(FULL, fabsf(gal16.x) < 1.0e7f && fabsf(gal16.y) < 1.0e7f && gMax < 9.0e8f)) {
 #pragma unroll
-      for (int u = 0; u < PER; ++u) {
-        const uint32_t k = (uint32_t)(u * NT + tid);
-        if (k < nb) {
-          s_id[k] = pf[u];
-          cp_async_rec(&s_rec[k], recs + pf[u]);
-        }
+        for (int k = 0; k < 10; ++k)
+          xs[k] = make_float2(fminf(fmaxf(xs[k].x, -1.0e9f), 1.0e9f), fminf(fmaxf(xs[k].y, -1.0e9f), 1.0e9f));
       }
-      cp_async_commit();
-      if (lo > 0) load_ids(s + lo_of(lo), s + lo);
-      cp_async_wait<0>();
-      __syncthreads();
-      {
-        const RenderRec* srec = s_rec;
-        for (int32_t w = (int32_t)((hi - 1) >> 5); w >= (int32_t)(lo >> 5); --w) {
-          const uint32_t wb = (uint32_t)w << 5;
-          uint32_t word = (uint32_t)w < (uint32_t)MASKW ? wmask[w] : FULL;
-          if (wb + 32u > hi) word &= FULL >> (wb + 32u - hi);
-          if (wb < lo) word &= FULL << (lo - wb);
-          while (word) {
-            const uint32_t bit = 31u - (uint32_t)__clz(word);
-            word &= ~(1u << bit);
-            const uint32_t j = wb + bit;
-            const RenderRec& rr = srec[j - lo];
-            const float4 r0 = rr.r0;
-            const float4 r1 = rr.r1;
-            const float4 r2 = rr.r2;
-            const float dx = px - r0.x;
-            const float2 dy = __fadd2_rn(py, bc2(-r0.y));
-            float2 Bdy;
-            const float2 ee = pairExponent2(r0, r1.x, dx, dy, Bdy);
-            const float2 G = gexp2(make_float2(-fminf(ee.x, 80.0f), -fminf(ee.y, 80.0f)));
-            const float2 araw = __fmul2_rn(bc2(r1.y), G);
-            const float2 alpha = make_float2(fminf(0.99f, araw.x), fminf(0.99f, araw.y));
-            const bool c2a = j < myEndA && ee.x <= E_CUT && alpha.x >= A_MIN;
-            const bool c2b = j < myEndB && ee.y <= E_CUT && alpha.y >= A_MIN;
-            const uint32_t balA = __ballot_sync(FULL, c2a), balB = __ballot_sync(FULL, c2b);
-            if ((balA | balB) == 0u) continue;
-            const float2 inv = rcp_unit2(__fadd2_rn(bc2(1.0f), make_float2(-alpha.x, -alpha.y)));
-            const float2 Tb = __fmul2_rn(Ta, inv);
-            const float2 at = __fmul2_rn(alpha, Tb);
-            const float2 aT = make_float2(c2a ? at.x : 0.0f, c2b ? at.y : 0.0f);
-            const float2 g0 = __ffma2_rn(bc2(r1.z), Tb, __fmul2_rn(make_float2(-S0.x, -S0.y), inv));
-            const float2 g1 = __ffma2_rn(bc2(r1.w), Tb, __fmul2_rn(make_float2(-S1.x, -S1.y), inv));
-            const float2 g2 = __ffma2_rn(bc2(r2.x), Tb, __fmul2_rn(make_float2(-S2.x, -S2.y), inv));
-            // galpha * 2^14, accumulated from gC * 2^14
-            const float2 gal16r = __ffma2_rn(g16_2, g2, __ffma2_rn(g16_1, g1, __fmul2_rn(g16_0, g0)));
-            const float2 gal16 = make_float2(c2a && !(araw.x > 0.99f) ? gal16r.x : 0.0f,
-                                             c2b && !(araw.y > 0.99f) ? gal16r.y : 0.0f);
-            const float2 ga16 = __fmul2_rn(gal16, araw);
-            const float cA = r0.z + r0.z, cC = r1.x + r1.x;
-            const float2 gq16 = __fmul2_rn(ga16, bc2(r2.z));
-            const float2 gqx16 = __fmul2_rn(gq16, bc2(dx));
-            float2 xs[10];
-            xs[0] = __fmul2_rn(ga16, __ffma2_rn(bc2(cA), bc2(dx), Bdy));
-            xs[1] = __fmul2_rn(ga16, __ffma2_rn(bc2(r0.w), bc2(dx), __fmul2_rn(bc2(cC), dy)));
-            xs[2] = __fmul2_rn(gqx16, bc2(dx));
-            xs[3] = __fmul2_rn(__fmul2_rn(gqx16, dy), bc2(2.0f));
-            xs[4] = __fmul2_rn(__fmul2_rn(gq16, dy), dy);
-            xs[5] = __fmul2_rn(__fmul2_rn(gal16, bc2(r2.y)), G);
-            xs[6] = __fmul2_rn(ga16, bc2(r2.w));
-            xs[7] = __fmul2_rn(g16_0, aT);
-            xs[8] = __fmul2_rn(g16_1, aT);
-            xs[9] = __fmul2_rn(g16_2, aT);
-            uint32_t rsum[10];
-            if (!__all_sync(FULL, fabsf(gal16.x) < 1.0e7f && fabsf(gal16.y) < 1.0e7f && pixFast)) {
+      S0 = __ffma2_rn(bc2(r1.z), aT, S0);
+      S1 = __ffma2_rn(bc2(r1.w), aT, S1);
+      S2 = __ffma2_rn(bc2(r2.x), aT, S2);
+      Ta = Tb;
+      // the 10 sums (every lane has them) go through shared memory, and lanes
+      // 0-9 add one each to the splat's slots; two staging rows in turn, so
+      // one barrier an entry is enough
+      int32_t q[10];
 #pragma unroll
-              for (int k = 0; k < 10; ++k)
-                xs[k] = make_float2(fminf(fmaxf(xs[k].x, -1.0e9f), 1.0e9f), fminf(fmaxf(xs[k].y, -1.0e9f), 1.0e9f));
-            }
-            // a half of the block with no compositing pixel has every value 0
-            if (balA != 0u && balB != 0u) {
-#pragma unroll
-              for (int k = 0; k < 10; ++k)
-                rsum[k] = __reduce_add_sync(FULL, (uint32_t)__float2int_rz(xs[k].x) + (uint32_t)__float2int_rz(xs[k].y));
-            } else if (balA != 0u) {
-#pragma unroll
-              for (int k = 0; k < 10; ++k) rsum[k] = __reduce_add_sync(FULL, (uint32_t)__float2int_rz(xs[k].x));
-            } else {
-#pragma unroll
-              for (int k = 0; k < 10; ++k) rsum[k] = __reduce_add_sync(FULL, (uint32_t)__float2int_rz(xs[k].y));
-            }
-            // a pixel that does not composite has aT = 0: S stays exactly as it is
-            S0 = __ffma2_rn(bc2(r1.z), aT, S0);
-            S1 = __ffma2_rn(bc2(r1.w), aT, S1);
-            S2 = __ffma2_rn(bc2(r2.x), aT, S2);
-            Ta = make_float2(c2a ? Tb.x : Ta.x, c2b ? Tb.y : Ta.y);
-            if (lane == 0) {
-              int4* st = reinterpret_cast<int4*>(s_stage[wid]);
-              st[0] = make_int4((int)rsum[0], (int)rsum[1], (int)rsum[2], (int)rsum[3]);
-              st[1] = make_int4((int)rsum[4], (int)rsum[5], (int)rsum[6], (int)rsum[7]);
-              reinterpret_cast<int2*>(s_stage[wid])[4] = make_int2((int)rsum[8], (int)rsum[9]);
-            }
-            __syncwarp();
-            if (lane < 10) atomicAdd(&s_acc[(j - lo) * 10 + (uint32_t)lane], s_stage[wid][lane]);
-            __syncwarp();
-          }
+      for (int k = 0; k < 10; ++k) q[k] = __float2int_rz(xs[k].x) + __float2int_rz(xs[k].y);
+      sts4(row, __reduce_add_sync(FULL, q[0]), __reduce_add_sync(FULL, q[1]), __reduce_add_sync(FULL, q[2]),
+           __reduce_add_sync(FULL, q[3]));
+      sts4(row + 16, __reduce_add_sync(FULL, q[4]), __reduce_add_sync(FULL, q[5]), __reduce_add_sync(FULL, q[6]),
+           __reduce_add_sync(FULL, q[7]));
+      sts2(row + 32, __reduce_add_sync(FULL, q[8]), __reduce_add_sync(FULL, q[9]));
+      __syncwarp();
+      // lanes from 10 on read word 10, which stays 0
+      red_nz(gradP + (size_t)lds1(sr + 48) * GP_STRIDE, (int32_t)lds1(row + slotOff));
+      row ^= 64u;
+    };
+    // list entries past the cache: recompute the exponentials chunk by chunk
+    if (uncached < e) {
+      const uint32_t endA = inA ? cntA : 0u, endB = inB ? cntB : 0u;
+      for (uint32_t base = seenEnd; base > uncached;) {  // both a whole number of chunks after s
+        base -= 32;
+        const uint32_t bits = stage(base + lane < e ? a.ids[base + lane] : 0u, base + lane < e, 0);
+        cp_async_wait<0>();
+        __syncwarp();
+        widen(s_rec[wid][0], (uint32_t)__popc(bits));
+        for (int k = __popc(bits) - 1; k >= 0; --k) {
+          const StagedRec* sr = &s_rec[wid][0][k];
+          const uint32_t j = base - s + sr->raw;
+          const float dx = px - sr->rec.r0.x;
+          const float2 dy = __fadd2_rn(py, bc2(-sr->rec.r0.y));
+          float2 Bdy;
+          const float2 ee = pairExponent2(sr->rec.r0, sr->rec.r1.x, dx, dy, Bdy);
+          const float2 G = gexp2(make_float2(-ee.x, -ee.y));
+          const float2 araw = __fmul2_rn(bc2(sr->rec.r1.y), G);
+          const bool c2a = j < endA && ee.x <= E_CUT && araw.x >= A_MIN;
+          const bool c2b = j < endB && ee.y <= E_CUT && araw.y >= A_MIN;
+          if (__any_sync(FULL, c2a || c2b))
+            backward(smem_addr(sr), make_float2(c2a ? G.x : 0.0f, c2b ? G.y : 0.0f), std::false_type{});
         }
-        __syncthreads();
-        for (uint32_t k = tid; k < nb * 10; k += NT) {
-          const int32_t val = s_acc[k];
-          if (val) {
-            const uint32_t jl = k / 10, slot = k - jl * 10;
-            atomicAdd(&gradP[(size_t)s_id[jl] * GP_STRIDE + slot], val);
-            s_acc[k] = 0;
-          }
-        }
+        __syncwarp();
       }
-      hi = lo;
     }
+    // cached entries, back to front, 32 records at a time; the exponentials
+    // load two entries ahead (they mostly come from DRAM)
+    const uint32_t vis = (uint32_t)((gp - gFirst) >> 5);
+    if (vis) {
+      const float2* gl = gp - 32;
+      float2 G0 = __ldcg(gl), G1 = __ldcg(gl - 32);  // this entry's exponentials and the next one's
+      auto stage_cached = [&](uint32_t hi, int b) {  // entries [max(hi - 32, 0), hi): lane l holds entry hi - 1 - l
+        if ((uint32_t)lane < hi) {
+          const uint32_t id = __ldcg(cacheId + (hi - 1 - lane));
+          s_rec[wid][b][lane].id = id;
+          cp_async_rec(&s_rec[wid][b][lane].rec, recs + id);
+        }
+        cp_async_commit();
+      };
+      int b = 0;
+      __syncwarp();
+      stage_cached(vis, 0);
+      for (uint32_t hi = vis; hi > 0;) {
+        const uint32_t n = hi < 32u ? hi : 32u;
+        if (hi > 32u) {
+          stage_cached(hi - 32u, b ^ 1);
+          cp_async_wait<1>();
+        } else {
+          cp_async_wait<0>();
+        }
+        __syncwarp();
+        const StagedRec* sr = s_rec[wid][b];
+        widen(sr, n);
+        auto chunk = [&](auto FAST) {
+          uint32_t at = smem_addr(sr);
+          for (const uint32_t end = at + n * (uint32_t)sizeof(StagedRec); at != end; at += (uint32_t)sizeof(StagedRec)) {
+            const float2 G = G0;
+            G0 = G1;
+            G1 = __ldcg(gl - 64);
+            gl -= 32;
+            backward(at, G, FAST);
+          }
+        };
+        if (fast) chunk(std::true_type{});
+        else chunk(std::false_type{});
+        __syncwarp();
+        hi -= n;
+        b ^= 1;
+      }
+    }
+  }
+  if (BWD) {
     __syncthreads();
+    if (threadIdx.x < 3 && s_stat[threadIdx.x]) atomicAdd(&a.stats[threadIdx.x], s_stat[threadIdx.x]);
+    if (threadIdx.x < 2 * a.V) {
+      const int v = threadIdx.x >> 1, k = threadIdx.x & 1;
+      if (s_cam[v][k]) atomicAdd(&a.gradCam[a.cams[v].camIdx * 8u + 6u + (uint32_t)k], s_cam[v][k]);
+    }
   }
 }
 
-template <int TILE, int BATCH, bool FWD, bool BWD, bool STORED>
-static void launch_one(const RasterArgs& a, unsigned grid, cudaStream_t s) {
-  if constexpr (TILE == 16 && FWD && BWD && !STORED) k_raster_px2<BATCH><<<grid, 128, 0, s>>>(a);
-  else k_raster<TILE, BATCH, FWD, BWD, STORED><<<grid, TILE * TILE, 0, s>>>(a);
-}
-
-template <int TILE, int BATCH>
-static void launch_mode(const RasterArgs& a, int mode, bool stored, unsigned grid, cudaStream_t s) {
-  // mode: 1 = forward, 2 = backward from saved state, 3 = fused train tile
-  if (mode == 1) launch_one<TILE, BATCH, true, false, false>(a, grid, s);
-  else if (mode == 2) {
-    if (stored) launch_one<TILE, BATCH, false, true, true>(a, grid, s);
-    else launch_one<TILE, BATCH, false, true, false>(a, grid, s);
-  } else {
-    if (stored) launch_one<TILE, BATCH, true, true, true>(a, grid, s);
-    else launch_one<TILE, BATCH, true, true, false>(a, grid, s);
-  }
+// wide: the build with more registers a thread, for grids of at most 5 blocks per SM
+static const void* warp_kernel(int tile, bool masked, bool train, bool wide) {
+  if (tile == 8) return train ? (const void*)k_raster_warp<8, false, true, 6> : (const void*)k_raster_warp<8, false, false, 8>;
+  if (tile == 32)
+    return train ? (const void*)k_raster_warp<32, false, true, 6> : (const void*)k_raster_warp<32, false, false, 8>;
+  if (!masked)
+    return train ? (const void*)k_raster_warp<16, false, true, 6> : (const void*)k_raster_warp<16, false, false, 8>;
+  if (!train) return (const void*)k_raster_warp<16, true, false, 8>;
+  return wide ? (const void*)k_raster_warp<16, true, true, 5> : (const void*)k_raster_warp<16, true, true, 7>;
 }
 
 template <int TILE>
-static void launch_tile(const RasterArgs& a, int mode, bool stored, int batchDepth, unsigned grid, cudaStream_t s) {
+static void launch_stored(const RasterArgs& a, int batchDepth, unsigned grid, cudaStream_t s) {
   switch (batchDepth) {
-    case 64: launch_mode<TILE, 64>(a, mode, stored, grid, s); break;
-    case 128: launch_mode<TILE, 128>(a, mode, stored, grid, s); break;
-    default: launch_mode<TILE, 256>(a, mode, stored, grid, s); break;
+    case 64: k_raster_stored<TILE, 64><<<grid, TILE * TILE, 0, s>>>(a); break;
+    case 128: k_raster_stored<TILE, 128><<<grid, TILE * TILE, 0, s>>>(a); break;
+    default: k_raster_stored<TILE, 256><<<grid, TILE * TILE, 0, s>>>(a); break;
   }
 }
 
-void launch_raster(const RasterArgs& a, int mode, bool stored, int tile, int batchDepth, unsigned grid,
-                   cudaStream_t s) {
+void launch_raster_stored(const RasterArgs& a, int tile, int batchDepth, unsigned grid, cudaStream_t s) {
   if (grid == 0) return;
-  if (tile == 8) launch_tile<8>(a, mode, stored, batchDepth, grid, s);
-  else if (tile == 32) launch_tile<32>(a, mode, stored, batchDepth, grid, s);
-  else launch_tile<16>(a, mode, stored, batchDepth, grid, s);
+  if (tile == 8) launch_stored<8>(a, batchDepth, grid, s);
+  else if (tile == 32) launch_stored<32>(a, batchDepth, grid, s);
+  else launch_stored<16>(a, batchDepth, grid, s);
 }
 
-// The kernel launch_one runs for (TILE, depth, forward-only or fused train
-// tile, not stored) and its block size.
-template <int TILE, int BATCH>
-static const void* kernel_of_depth(bool fwdOnly, int& threads) {
-  threads = TILE * TILE;
-  if (fwdOnly) return (const void*)k_raster<TILE, BATCH, true, false, false>;
-  if (TILE == 16) {
-    threads = 128;
-    return (const void*)k_raster_px2<BATCH>;
+void launch_raster(const RasterArgs& a, bool train, int tile, unsigned grid, int sms, cudaStream_t s) {
+  if (grid == 0) return;
+  RasterArgs copy = a;
+  void* args[] = {&copy};
+  cudaLaunchKernel(warp_kernel(tile, a.idMask != 0xFFFFFFFFu, train, grid <= 5u * (unsigned)sms), dim3(grid),
+                   dim3(RW_WARPS * 32), args, 0, s);
+}
+
+int raster_blocks_per_sm(int tile, bool train) {
+  int least = 64;
+  for (int k = 0; k < 4; ++k) {
+    if (k == 3 && train) continue;  // the wide build runs on smaller grids only
+    int n = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, warp_kernel(tile, (k & 1) != 0, train, (k & 2) != 0),
+                                                  RW_WARPS * 32, 0);
+    if (n < least) least = n;
   }
-  return (const void*)k_raster<TILE, BATCH, true, true, false>;
+  return least < 1 ? 1 : least;
 }
 
-template <int TILE>
-static const void* kernel_of(int batchDepth, int mode, int& threads) {
-  const bool fwdOnly = mode == 1;
-  switch (batchDepth) {
-    case 64: return kernel_of_depth<TILE, 64>(fwdOnly, threads);
-    case 128: return kernel_of_depth<TILE, 128>(fwdOnly, threads);
-    default: return kernel_of_depth<TILE, 256>(fwdOnly, threads);
-  }
-}
-
-int raster_blocks_per_sm(int tile, int batchDepth, int mode) {
-  int threads = 0;
-  const void* f = tile == 8 ? kernel_of<8>(batchDepth, mode, threads)
-                            : tile == 32 ? kernel_of<32>(batchDepth, mode, threads)
-                                         : kernel_of<16>(batchDepth, mode, threads);
-  int perSm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, f, threads, 0);
-  return perSm < 1 ? 1 : perSm;
+// Blocks of the persistent raster over `items` 8x8 blocks.  The longest tiles
+// are taken first, and with every warp slot filled they share an SM with 27
+// others and finish last, so when there are only a few items per slot fewer
+// blocks are launched: about 5.3 items a warp, at least 3 blocks per SM.
+// Train passes at 7 / 6 / 5 / 4 / 3 blocks per SM, us a pass: 3780 items
+// 8995 / 8938 / 8696 / 8218 / 7797; 10032 items 14020 / 13801 / 13211 / 12582 /
+// 12827; 15504 items 8870 / 8734 / 8452 / 8601 / 9325; 32640 items 47788 /
+// 48405 / 50258 / 53515 / 58853.
+unsigned raster_grid(uint32_t items, int sms, int perSm) {
+  const unsigned all = (items + RW_WARPS - 1) / RW_WARPS;
+  const double k = std::ceil((double)items / (5.3 * RW_WARPS * sms));
+  const unsigned blocks = (unsigned)(std::min((double)perSm, std::max(3.0, k)) * sms);
+  return all < blocks ? all : blocks;
 }
 
 // Work order for the persistent queue: global tiles by descending entry

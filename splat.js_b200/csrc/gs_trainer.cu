@@ -125,6 +125,7 @@ struct gs_trainer {
   int lastV = 0;
   DevCam lastCams[MAXB];
   int lastPasses = 0;
+  bool lastMasks = false;  // entry values carry block bits
   uint32_t lastLaunches = 0;
   uint32_t lastTotalTiles = 0;
 
@@ -140,7 +141,10 @@ struct gs_trainer {
   std::map<Shape, cudaGraphExec_t> graphs;
   int histGrid = 0, sweepGrid = 0;
   int tile = 16;                 // current raster tile edge (8, 16 or 32)
-  int rasterPerSm[3][3][2] = {};  // occupancy per (tile, batch depth, forward-only / train)
+  int rasterPerSm[3][2] = {};    // occupancy per (tile, forward-only / train)
+  float2* cacheG = nullptr;      // the raster's exponential cache (train passes), see RasterArgs
+  uint32_t* cacheId = nullptr;
+  uint32_t cacheCap = 0, cacheWarps = 0;
 
   // ---- measurement ----
   cudaStream_t ownStream = nullptr;
@@ -311,9 +315,7 @@ int gs_create(const gs_options* opts, gs_trainer** out) {
   h->sweepGrid = onesweep_grid(h->device);
   h->tile = o.tile;
   for (int ti = 0; ti < 3; ++ti)
-    for (int di = 0; di < 3; ++di)
-      for (int m = 0; m < 2; ++m)
-        h->rasterPerSm[ti][di][m] = raster_blocks_per_sm(8 << ti, 64 << di, m == 0 ? 1 : 3);
+    for (int m = 0; m < 2; ++m) h->rasterPerSm[ti][m] = raster_blocks_per_sm(8 << ti, m == 1);
   *out = h;
   return GS_OK;
 }
@@ -436,6 +438,21 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
   GS_AL(h->shGradOut, std::max<size_t>(shn, 1));
   GS_AL(h->dParams, (size_t)1);
 #undef GS_AL
+  {  // the raster's exponential cache; without memory for it every entry is recomputed
+    const int perSm = std::max(std::max(h->rasterPerSm[0][1], h->rasterPerSm[1][1]), h->rasterPerSm[2][1]);
+    uint32_t blocks = ceil_div(maxViewW, 32) * ceil_div(maxViewH, 32);  // of 32 pixels, the largest tile
+    for (uint32_t c = 0; c < ncams; ++c)
+      blocks = std::max(blocks, ceil_div((uint32_t)h->cams[c].w, 32) * ceil_div((uint32_t)h->cams[c].h, 32));
+    h->cacheWarps = (uint32_t)std::min<uint64_t>((uint64_t)h->sms * perSm * RW_WARPS,
+                                                 std::max<uint64_t>((uint64_t)B * blocks * 16, RW_WARPS));
+    h->cacheCap = RASTER_CACHE_ENTRIES;
+    if (dalloc(h, &h->cacheG, ((size_t)h->cacheWarps * (h->cacheCap + 2) + 1) * 32) != GS_OK) {
+      cudaGetLastError();  // not an error: one slot a warp is enough to run
+      h->cacheCap = 0;
+      if ((rc = dalloc(h, &h->cacheG, ((size_t)h->cacheWarps * 2 + 1) * 32)) != GS_OK) { free_all(h); return rc; }
+    }
+    if ((rc = dalloc(h, &h->cacheId, (size_t)h->cacheWarps * (h->cacheCap + 2))) != GS_OK) { free_all(h); return rc; }
+  }
   if (cudaMallocHost(&h->hRing, sizeof(StepParams) * RING) != cudaSuccess) {
     free_all(h);
     return fail(h, GS_E_NOMEM, "cudaMallocHost(step parameters) failed");
@@ -577,6 +594,10 @@ static int upload_params(gs_trainer* h, const DevCam* views, int V, const AdamHP
   return k;
 }
 
+// Entry values carry 8x8 block bits above the splat id (k_expand) when the
+// tile is 16 pixels (four blocks) and the ids leave four bits free.
+static bool block_masks(int tile, uint32_t n) { return tile == 16 && n <= (1u << ID_BITS); }
+
 // Enqueues project -> bin -> sort -> raster [-> chain/Adam] for the views
 // whose records were uploaded last.  All sizes the device decides (entry
 // counts) are read on the device, so the sequence can be captured.
@@ -677,6 +698,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   const uint32_t* sortedSlots = h->pvals[pr.passes & 1];
 
   const bool cull = sh.cull != 0;
+  const bool masks = block_masks(sh.tile, sh.n);
   ExpandArgs ea{};
   ea.n = sh.n;
   ea.V = V;
@@ -691,6 +713,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   ea.aMin = h->o.aMin;
   ea.tile = sh.tile;
   ea.cull = cull ? 1 : 0;
+  ea.masks = masks ? 1 : 0;
   ea.counts = h->counts;
   ea.offsets = h->offsets;
   ea.keys = h->keys[0];
@@ -723,6 +746,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   ra.sweepGrid = (unsigned)h->sweepGrid;
   launch_radix_sort(ra, s);
   h->lastPasses = passes;
+  h->lastMasks = masks;
   if (cull) launch_ranges_from_keys(h->keys[passes & 1], totalEntries, totalTiles, h->ranges, s);
   // kernels: project, tile counts + finish, presort (histogram + passes),
   // entry counts, 3 scan kernels, entry keys, tile sort (histogram +
@@ -741,6 +765,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   rr.recs = h->recs;
   rr.cullRecs = h->cullRecs;
   rr.ids = sortedIds;
+  rr.idMask = masks ? ID_MASK : 0xFFFFFFFFu;
   rr.ranges = h->ranges;
   rr.totalTiles = totalTiles;
   rr.workOrder = persistent ? h->workOrder : nullptr;
@@ -755,14 +780,22 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   rr.stats = h->stats;
   rr.gradCam = h->gradCam;
   rr.tStore = h->tStore;
-  unsigned grid = totalTiles;
-  if (persistent) {
-    const int ti = sh.tile == 8 ? 0 : sh.tile == 16 ? 1 : 2;
-    const int di = sh.depth == 64 ? 0 : sh.depth == 128 ? 1 : 2;
-    const unsigned full = (unsigned)(h->sms * h->rasterPerSm[ti][di][sh.mode == 1 ? 0 : 1]);
-    grid = std::min(grid, full);
+  const bool train = sh.mode == 3;
+  rr.cacheG = h->cacheG;
+  rr.cacheId = h->cacheId;
+  rr.cacheWarps = h->cacheWarps;
+  rr.cacheCap = persistent ? h->cacheCap : 0u;  // one block a tile: no slice of a warp's own
+  const int perSm = h->rasterPerSm[sh.tile == 8 ? 0 : sh.tile == 16 ? 1 : 2][train ? 1 : 0];
+  if (train && sh.variant == 1) {
+    launch_raster_stored(rr, sh.tile, sh.depth,
+                         persistent ? std::min(totalTiles, (uint32_t)(h->sms * perSm)) : totalTiles, s);
+  } else {  // one warp per 8x8 block of a tile
+    const uint32_t rasterItems = totalTiles * (uint32_t)((sh.tile / 8) * (sh.tile / 8));
+    unsigned grid = ceil_div(rasterItems, RW_WARPS);
+    if (persistent) grid = raster_grid(rasterItems, h->sms, perSm);
+    if (persistent && train) grid = std::min(grid, h->cacheWarps / RW_WARPS);  // a slice for every warp
+    launch_raster(rr, train, sh.tile, grid, h->sms, s);
   }
-  launch_raster(rr, sh.mode, sh.variant == 1, sh.tile, sh.depth, grid, s);
   if (h->profiling) cudaEventRecord(ph[3], s);
 
   if (sh.chain) {
@@ -1190,6 +1223,8 @@ int gs_debug_binning(gs_trainer* h, uint32_t view, uint32_t* tileCnt, uint32_t* 
     const uint64_t k = std::min<uint64_t>(cap, E);
     GS_CK(cudaMemcpyAsync(ids, h->vals[h->lastPasses & 1], k * 4, cudaMemcpyDeviceToHost, h->stream));
     GS_CK(cudaStreamSynchronize(h->stream));
+    if (h->lastMasks)
+      for (uint64_t i = 0; i < k; ++i) ids[i] &= ID_MASK;
   }
   return GS_OK;
 }
