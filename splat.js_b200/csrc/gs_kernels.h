@@ -15,6 +15,18 @@ namespace gs {
 // sums: the counts do not depend on the split.
 constexpr uint32_t GRID_COPIES = 4;
 
+// First kernel of a pass (k_step_begin).
+struct StepBeginArgs {
+  const uint32_t* ring;    // pinned host memory: `slots` parameter records of `words` words
+  uint32_t slots, words;
+  uint32_t* seq;           // passes run so far: this one takes slot seq % slots
+  uint32_t* params;        // device copy of the record
+  uint32_t* nItems;        // presort items of the pass, set to `items`
+  uint32_t items;
+  uint32_t* clear[3];      // word ranges set to zero
+  uint32_t count[3];
+};
+
 struct ProjectArgs {
   const float* params;     // n * 16
   const float* sh;         // n * 3K (channel-major) or null
@@ -42,7 +54,7 @@ struct TileRangeArgs {
   uint32_t gridCells;
   uint32_t* tileCnt;       // per global tile: the reference's tileCnt
   uint8_t* dropped;        // per global tile: dropped by the entry budget
-  uint2* ranges;           // per global tile: [start, end) in the sorted entries
+  uint2* ranges;           // per global tile: [start, end) in the sorted entries, or null: not wanted
   uint32_t* viewDrops;     // per view: number of dropped tiles
   uint32_t* viewTotal;     // per view: kept entries
   uint32_t* stats;         // stats[3] += dropped tiles
@@ -220,6 +232,7 @@ struct RefineApplyArgs {
 };
 
 // launchers
+void launch_step_begin(const StepBeginArgs& a, cudaStream_t s);
 void launch_project(const ProjectArgs& a, int deg, cudaStream_t s);
 void launch_tile_ranges(const TileRangeArgs& a, uint32_t totalTiles, cudaStream_t s);
 void launch_expand(const ExpandArgs& a, bool keys, cudaStream_t s);

@@ -27,6 +27,32 @@
 
 namespace gs {
 
+// Starts a pass: block 0 fetches the pass's parameter record straight from the
+// pinned host ring (the kernels after it read the device copy), and the grid
+// clears the pass's counters.  As one kernel in front it replaces a copy
+// outside the graph and five memset and two copy nodes in it; between kernel
+// nodes the gap is 0.2 us, around memset nodes 2.5-8 us.  Bound by the PCIe
+// round trip of the record (2.2 KB).
+__global__ void __launch_bounds__(256) k_step_begin(StepBeginArgs a) {
+  if (blockIdx.x == 0) {
+    const uint32_t* src = a.ring + (size_t)(*a.seq % a.slots) * a.words;
+    for (uint32_t k = threadIdx.x; k < a.words; k += blockDim.x) {
+      uint32_t w;  // written by the host before the launch: not from a cache
+      asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(w) : "l"(src + k));
+      a.params[k] = w;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      *a.seq += 1u;
+      *a.nItems = a.items;
+    }
+  }
+  const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+    for (uint32_t k = at; k < a.count[r]; k += stride) a.clear[r][k] = 0u;
+}
+
 // One thread per splat, looping over the batch's views: parameters and SH
 // coefficients are read once per step.
 template <int DEG>
@@ -227,6 +253,7 @@ __global__ void __launch_bounds__(1024) k_tile_counts(TileRangeArgs a) {
   if (!anyDrop)
     for (int t = threadIdx.x; t < nt; t += blockDim.x) dr[t] = 0;
   __syncthreads();
+  if (!a.ranges) return;
   // exclusive scan of kept counts in tile order -> view-local ranges
   const int per = (nt + blockDim.x - 1) / blockDim.x;
   const int t0 = threadIdx.x * per;
@@ -560,6 +587,12 @@ __global__ void __launch_bounds__(256) k_ranges_from_keys(const uint32_t* keys, 
   ranges[gt] = make_uint2(lower_bound_u32(keys, E, gt), lower_bound_u32(keys, E, gt + 1));
 }
 
+void launch_step_begin(const StepBeginArgs& a, cudaStream_t s) {
+  uint32_t words = 0;
+  for (int r = 0; r < 3; ++r) words = a.count[r] > words ? a.count[r] : words;
+  const unsigned blocks = (words + 1023) / 1024;  // four words a thread
+  k_step_begin<<<blocks < 296 ? (blocks ? blocks : 1) : 296, 256, 0, s>>>(a);
+}
 void launch_project(const ProjectArgs& a, int deg, cudaStream_t s) {
   const unsigned grid = (a.n + 255) / 256;
   if (grid == 0) return;
@@ -572,7 +605,7 @@ void launch_project(const ProjectArgs& a, int deg, cudaStream_t s) {
 }
 void launch_tile_ranges(const TileRangeArgs& a, uint32_t totalTiles, cudaStream_t s) {
   k_tile_counts<<<a.V, 1024, 0, s>>>(a);
-  k_tile_ranges_finish<<<(totalTiles + 255) / 256, 256, 0, s>>>(a, totalTiles);
+  if (a.ranges) k_tile_ranges_finish<<<(totalTiles + 255) / 256, 256, 0, s>>>(a, totalTiles);
 }
 void launch_expand(const ExpandArgs& a, bool keys, cudaStream_t s) {
   const uint64_t total = (uint64_t)a.n * a.V;

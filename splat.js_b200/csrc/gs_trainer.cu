@@ -25,13 +25,14 @@ namespace {
 
 constexpr int MAXB = MAX_VIEWS;  // hard upper bound of views per batch
 constexpr int RING = 8;      // pinned step-parameter slots
+constexpr int SMALL_SEQ = 2200;  // word of `small` that counts the passes run
 
 struct StepParams {
   AdamHP hp;
   uint32_t gridBase[MAXB];
-  uint32_t itemCount;        // V * n presort items of this step
   DevCam cams[MAXB];
 };
+static_assert(sizeof(StepParams) % 4 == 0, "step parameters are copied as words");
 
 thread_local std::string g_createError;
 
@@ -118,7 +119,11 @@ struct gs_trainer {
   StepParams* dParams = nullptr;
   StepParams* hRing = nullptr;
   cudaEvent_t ringEv[RING] = {};
-  int ringPos = 0;
+  uint32_t seq = 0;              // passes enqueued: the next one reads slot seq % RING (k_step_begin)
+  bool filled = false;           // that slot holds the next pass's parameters
+  bool seqLost = false;          // an enqueue failed: the device's count may differ from seq
+  cudaStream_t side = nullptr;   // second branch of the captured step
+  cudaEvent_t forkEv = nullptr, joinEv = nullptr;
   std::vector<void*> allocs;
 
   // ---- last raster (for introspection) ----
@@ -309,6 +314,13 @@ int gs_create(const gs_options* opts, gs_trainer** out) {
     return GS_E_CUDA;
   }
   for (int k = 0; k < RING; ++k) cudaEventCreateWithFlags(&h->ringEv[k], cudaEventDisableTiming);
+  if (cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->forkEv, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&h->joinEv, cudaEventDisableTiming) != cudaSuccess) {
+    g_createError = "cudaStreamCreate failed";
+    gs_destroy(h);
+    return GS_E_CUDA;
+  }
   h->K = o.shDeg > 0 ? (uint32_t)((o.shDeg + 1) * (o.shDeg + 1) - 1) : 0u;
   h->horizon = o.maxIters ? o.maxIters : 60000u;
   h->histGrid = h->sms * 4;
@@ -327,6 +339,9 @@ void gs_destroy(gs_trainer* h) {
   free_all(h);
   for (int k = 0; k < RING; ++k)
     if (h->ringEv[k]) cudaEventDestroy(h->ringEv[k]);
+  if (h->forkEv) cudaEventDestroy(h->forkEv);
+  if (h->joinEv) cudaEventDestroy(h->joinEv);
+  if (h->side) cudaStreamDestroy(h->side);
   cudaStream_t own = h->ownStream ? h->ownStream : h->stream;
   if (own) cudaStreamDestroy(own);
   delete h;
@@ -458,6 +473,8 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
     return fail(h, GS_E_NOMEM, "cudaMallocHost(step parameters) failed");
   }
   std::memset(h->hRing, 0, sizeof(StepParams) * RING);
+  h->seq = 0;
+  h->filled = h->seqLost = false;
   cudaStream_t s = h->stream;
   GS_CK(cudaMemcpyAsync(h->params, params, (size_t)n * 64, cudaMemcpyHostToDevice, s));
   GS_CK(cudaMemsetAsync(h->m, 0, cap * 64, s));
@@ -568,15 +585,13 @@ static int bits_for(uint32_t x) {  // bits needed to hold values 0..x
   return b;
 }
 
-// Fills a ring slot with the views' records and the Adam parameters and
-// queues its upload.  Returns the slot used.
-static int upload_params(gs_trainer* h, const DevCam* views, int V, const AdamHP& hp) {
-  const int k = h->ringPos;
-  h->ringPos = (h->ringPos + 1) % RING;
+// Fills the next ring slot with the views' records and the Adam parameters.
+// The pass that is enqueued next reads it on the device (k_step_begin).
+static void upload_params(gs_trainer* h, const DevCam* views, int V, const AdamHP& hp) {
+  const int k = (int)(h->seq % RING);
   cudaEventSynchronize(h->ringEv[k]);
   StepParams& P = h->hRing[k];
   P.hp = hp;
-  P.itemCount = (uint32_t)((uint64_t)V * h->n);
   uint32_t tb = 0, pb = 0, gb = 0;
   for (int v = 0; v < V; ++v) {
     P.cams[v] = views[v];
@@ -587,11 +602,31 @@ static int upload_params(gs_trainer* h, const DevCam* views, int V, const AdamHP
     pb += (uint32_t)(views[v].W * views[v].H);
     gb += (uint32_t)((views[v].tilesX + 1) * (views[v].tilesY + 1));
   }
-  cudaMemcpyAsync(h->dParams, &P, sizeof(StepParams), cudaMemcpyHostToDevice, h->stream);
-  cudaEventRecord(h->ringEv[k], h->stream);
+  h->filled = true;
   for (int v = 0; v < V; ++v) h->lastCams[v] = P.cams[v];
   h->lastV = V;
-  return k;
+}
+
+// Every pass enqueued consumes a slot.  A pass without parameters of its own
+// (a repeated one) runs with those of the pass before it.
+static int begin_pass(gs_trainer* h) {
+  if (h->seqLost) {
+    GS_CK(cudaStreamSynchronize(h->stream));
+    GS_CK(cudaMemcpy(h->small + SMALL_SEQ, &h->seq, 4, cudaMemcpyHostToDevice));
+    h->seqLost = false;
+  }
+  if (!h->filled) {
+    const int k = (int)(h->seq % RING);
+    cudaEventSynchronize(h->ringEv[k]);
+    h->hRing[k] = h->hRing[(h->seq + RING - 1) % RING];
+    h->filled = true;
+  }
+  return GS_OK;
+}
+static void end_pass(gs_trainer* h) {
+  cudaEventRecord(h->ringEv[h->seq % RING], h->stream);
+  ++h->seq;
+  h->filled = false;
 }
 
 // Entry values carry 8x8 block bits above the splat id (k_expand) when the
@@ -601,7 +636,9 @@ static bool block_masks(int tile, uint32_t n) { return tile == 16 && n <= (1u <<
 // Enqueues project -> bin -> sort -> raster [-> chain/Adam] for the views
 // whose records were uploaded last.  All sizes the device decides (entry
 // counts) are read on the device, so the sequence can be captured.
-static int enqueue_body(gs_trainer* h, const Shape& sh) {
+// fork: the tile counts run beside the presort on the second stream (for
+// capture; the events then become edges of the graph).
+static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   cudaStream_t s = h->stream;
   const int V = sh.V;
   uint32_t totalTiles = 0, gridCells = 0;
@@ -625,10 +662,28 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
     for (int k = 0; k < 5; ++k) cudaEventCreate(&ph[k]);
     cudaEventRecord(ph[0], s);
   }
-  cudaMemsetAsync(h->diffGrid, 0, (size_t)gridCells * GRID_COPIES * 4, s);
-  cudaMemsetAsync(h->small, 0, 2057 * 4, s);  // hist, tile counters, work counter
-  cudaMemsetAsync(h->small + 2062, 0, MAXB * 4, s);  // visible-item counters of the chain
   const uint64_t items = (uint64_t)sh.n * V;
+  const bool cull = sh.cull != 0;
+  const bool masks = block_masks(sh.tile, sh.n);
+  uint32_t* nItems = h->small + 2061;
+  uint32_t* liveItems = h->small + 2150;
+  {
+    StepBeginArgs ba{};
+    ba.ring = reinterpret_cast<const uint32_t*>(h->hRing);
+    ba.slots = RING;
+    ba.words = (uint32_t)(sizeof(StepParams) / 4);
+    ba.seq = h->small + SMALL_SEQ;
+    ba.params = reinterpret_cast<uint32_t*>(h->dParams);
+    ba.nItems = nItems;
+    ba.items = (uint32_t)items;
+    ba.clear[0] = reinterpret_cast<uint32_t*>(h->diffGrid);
+    ba.count[0] = gridCells * GRID_COPIES;
+    ba.clear[1] = h->small;  // histograms, block and work counters
+    ba.count[1] = 2057;
+    ba.clear[2] = h->small + 2062;  // visible-item counters, work order, live items
+    ba.count[2] = 2151 - 2062;
+    launch_step_begin(ba, s);
+  }
 
   ProjectArgs pa{};
   pa.params = h->params;
@@ -665,14 +720,18 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   ta.stats = h->stats;
   ta.entriesCap = h->entriesCap;
   ta.totalEntries = totalEntries;
-  launch_tile_ranges(ta, totalTiles, s);
+  ta.ranges = cull ? nullptr : h->ranges;  // culled lists take their ranges from the sorted keys
+  if (fork) {
+    cudaEventRecord(h->forkEv, s);
+    cudaStreamWaitEvent(h->side, h->forkEv, 0);
+  }
+  launch_tile_ranges(ta, totalTiles, fork ? h->side : s);
+  if (fork) cudaEventRecord(h->joinEv, h->side);
 
   // presort of the (view, splat) items by depth: 4 byte digits of the depth
   // bits, stable from slot order, so equal depths stay in splat order.  Views
   // stay interleaved: the tile sort groups entries by global tile id (which
   // belongs to one view) and keeps this order inside every tile.
-  uint32_t* nItems = h->small + 2061;
-  cudaMemcpyAsync(nItems, &h->dParams->itemCount, 4, cudaMemcpyDeviceToDevice, s);
   RadixSortArgs pr{};
   pr.keys[0] = h->pkeys[0]; pr.keys[1] = h->pkeys[1];
   pr.vals[0] = h->pvals[0]; pr.vals[1] = h->pvals[1];
@@ -690,15 +749,12 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   pr.sweepGrid = (unsigned)h->sweepGrid;
   // culled items (all-ones keys) leave the presort: only the visible ones
   // are sorted, and their count sizes the expansion
-  uint32_t* liveItems = h->small + 2150;
   pr.nKept = liveItems;
-  cudaMemsetAsync(liveItems, 0, 4, s);
   if (h->profiling) cudaEventRecord(ph[1], s);
   launch_radix_sort(pr, s);
   const uint32_t* sortedSlots = h->pvals[pr.passes & 1];
 
-  const bool cull = sh.cull != 0;
-  const bool masks = block_masks(sh.tile, sh.n);
+  if (fork) cudaStreamWaitEvent(s, h->joinEv, 0);  // the expansion reads the dropped tiles
   ExpandArgs ea{};
   ea.n = sh.n;
   ea.V = V;
@@ -721,21 +777,20 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   ea.capacity = h->capacity;
   ea.status = statusWord;
   launch_expand(ea, false, s);
-  launch_exclusive_scan(h->counts, items, h->offsets, h->scanPartials, scanTotal, s);
-  launch_expand(ea, true, s);
   // culled lists: the entry total is the counts' sum, not the budgeted tile sum
-  if (cull) cudaMemcpyAsync(totalEntries, scanTotal, 4, cudaMemcpyDeviceToDevice, s);
+  launch_exclusive_scan(h->counts, items, h->offsets, h->scanPartials, cull ? totalEntries : scanTotal, s);
+  launch_expand(ea, true, s);
 
-  // stable sort of the entries by global tile id
-  cudaMemsetAsync(h->small, 0, 2056 * 4, s);  // histograms and block counters of the second sort
+  // stable sort of the entries by global tile id: at most 4 passes, with
+  // histograms and block counters of its own behind the presort's four
   const int passes = (bits_for(totalTiles ? totalTiles - 1 : 0) + 7) / 8;
   RadixSortArgs ra{};
   ra.keys[0] = h->keys[0]; ra.keys[1] = h->keys[1];
   ra.vals[0] = h->vals[0]; ra.vals[1] = h->vals[1];
   ra.keyBytes = 4;
   ra.nItems = totalEntries;
-  ra.hist = hist;
-  ra.tileCounter = tileCounter;
+  ra.hist = hist + 4 * 256;
+  ra.tileCounter = tileCounter + 4;
   ra.status = h->lbStatus;
   ra.statusWord = statusWord;
   ra.epoch = epoch;
@@ -748,10 +803,10 @@ static int enqueue_body(gs_trainer* h, const Shape& sh) {
   h->lastPasses = passes;
   h->lastMasks = masks;
   if (cull) launch_ranges_from_keys(h->keys[passes & 1], totalEntries, totalTiles, h->ranges, s);
-  // kernels: project, tile counts + finish, presort (histogram + passes),
+  // kernels: begin, project, tile counts [+ finish], presort (histogram + passes),
   // entry counts, 3 scan kernels, entry keys, tile sort (histogram +
   // passes), [ranges from keys], [work order: 3], raster, [visible lists, chain per view, sum + Adam]
-  h->lastLaunches = 3u + 1u + (uint32_t)pr.passes + 1u + 3u + 1u + 1u + (uint32_t)passes + (cull ? 1u : 0u) +
+  h->lastLaunches = (cull ? 3u : 4u) + 1u + (uint32_t)pr.passes + 1u + 3u + 1u + 1u + (uint32_t)passes + (cull ? 1u : 0u) +
                     (h->o.persistent ? 3u : 0u) + 1u + (sh.chain ? 3u : 0u);
   const uint32_t* sortedIds = h->vals[passes & 1];
 
@@ -845,8 +900,10 @@ static int ensure_tstore(gs_trainer* h, const Shape& sh) {
   probe.mode = 1;
   probe.chain = 0;
   probe.variant = 0;
-  int rc = enqueue_body(h, probe);
+  int rc = begin_pass(h);
+  if (!rc) rc = enqueue_body(h, probe, false);
   if (rc) return rc;
+  end_pass(h);
   uint32_t E = 0;
   GS_CK(cudaMemcpyAsync(&E, h->small + 2057, 4, cudaMemcpyDeviceToHost, h->stream));
   GS_CK(cudaStreamSynchronize(h->stream));
@@ -866,17 +923,15 @@ static int ensure_tstore(gs_trainer* h, const Shape& sh) {
   return GS_OK;
 }
 
-static int run_shape(gs_trainer* h, const Shape& sh) {
-  if (sh.variant == 1) {
-    int rc = ensure_tstore(h, sh);
-    if (rc) return rc;
-  }
-  if (!h->o.useGraphs || sh.variant == 1 || h->profiling) return enqueue_body(h, sh);
+static int run_pass(gs_trainer* h, const Shape& sh) {
+  int rc = begin_pass(h);
+  if (rc) return rc;
+  if (!h->o.useGraphs || sh.variant == 1 || h->profiling) return enqueue_body(h, sh, false);
   auto it = h->graphs.find(sh);
   if (it == h->graphs.end()) {
     cudaGraph_t g = nullptr;
     GS_CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = enqueue_body(h, sh);
+    rc = enqueue_body(h, sh, true);
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (rc) { if (g) cudaGraphDestroy(g); return rc; }
     if (e != cudaSuccess) return fail(h, GS_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -887,6 +942,18 @@ static int run_shape(gs_trainer* h, const Shape& sh) {
     it = h->graphs.emplace(sh, ex).first;
   }
   GS_CK(cudaGraphLaunch(it->second, h->stream));
+  return GS_OK;
+}
+
+static int run_shape(gs_trainer* h, const Shape& sh) {
+  int rc = sh.variant == 1 ? ensure_tstore(h, sh) : GS_OK;
+  if (!rc) rc = run_pass(h, sh);
+  if (rc) {  // the device may or may not have counted this pass
+    h->seqLost = true;
+    h->filled = false;
+    return rc;
+  }
+  end_pass(h);
   return GS_OK;
 }
 
