@@ -60,7 +60,10 @@ struct TileRangeArgs {
   uint32_t* stats;         // stats[3] += dropped tiles
   uint64_t entriesCap;     // per-view entry budget (ENTCAP)
   uint32_t* totalEntries;  // out: kept entries over the batch
+  uint32_t* buckets;       // out: tiles per bucket (tile_bucket), zero before
 };
+
+constexpr uint32_t EXPAND_BLOCK = 256;  // presorted items per block of k_expand
 
 // Entry expansion of the presorted (view, depth, id) items (k_expand).
 struct ExpandArgs {
@@ -77,8 +80,8 @@ struct ExpandArgs {
   int tile;
   int cull;                     // 1: keep only entries tileLive() accepts
   int masks;                    // 1 (tile 16): entry values carry the 8x8 block bits
-  uint32_t* counts;             // count pass: V * n, in presorted order
-  const uint32_t* offsets;      // key pass: V * n exclusive scan of counts
+  uint32_t* counts;             // entries per presorted item (count pass -> key pass)
+  uint32_t* partials;           // entries per block of EXPAND_BLOCK items; scanned between the passes
   uint32_t* keys;               // global tile id per entry
   uint32_t* vals;               // entry value: splat id (and block bits)
   uint64_t capacity;
@@ -146,6 +149,9 @@ constexpr int RW_WARPS = 4;                    // warps per block of k_raster_wa
 #define GS_RASTER_CACHE 256  // composited entries a warp caches (k_raster_warp)
 #endif
 constexpr uint32_t RASTER_CACHE_ENTRIES = GS_RASTER_CACHE;
+
+// Work-order bucket of a tile: 32 empty, 0 longest.
+__device__ __forceinline__ uint32_t tile_bucket(uint2 r) { return (uint32_t)__clz((int)(r.y - r.x)); }
 
 struct RasterArgs {
   const DevCam* cams;
@@ -237,7 +243,8 @@ void launch_project(const ProjectArgs& a, int deg, cudaStream_t s);
 void launch_tile_ranges(const TileRangeArgs& a, uint32_t totalTiles, cudaStream_t s);
 void launch_expand(const ExpandArgs& a, bool keys, cudaStream_t s);
 void launch_ranges_from_keys(const uint32_t* keys, const uint32_t* nItems, uint32_t totalTiles, uint2* ranges,
-                             cudaStream_t s);
+                             uint32_t* buckets, cudaStream_t s);
+void launch_scan_blocks(uint32_t* partials, const uint32_t* nItems, uint32_t perBlock, uint32_t* total, cudaStream_t s);
 uint32_t scan_partials_needed(uint64_t N);
 void launch_exclusive_scan(const uint32_t* in, uint64_t N, uint32_t* out, uint32_t* partials, uint32_t* total,
                            cudaStream_t s);
@@ -254,8 +261,8 @@ void launch_raster(const RasterArgs& a, bool train, int tile, unsigned grid, int
 unsigned raster_grid(uint32_t items, int sms, int perSm);
 void launch_raster_stored(const RasterArgs& a, int tile, int batchDepth, unsigned grid, cudaStream_t s);
 int raster_blocks_per_sm(int tile, bool train);
-void launch_work_order(const uint2* ranges, uint32_t totalTiles, uint32_t* order, uint32_t* scratch,
-                       cudaStream_t s);
+void launch_work_place(const uint2* ranges, uint32_t totalTiles, const uint32_t* counts, uint32_t* cursors,
+                       uint32_t* order, cudaStream_t s);
 void launch_chain_adam(const ChainArgs& a, int deg, cudaStream_t s);
 void launch_refine_classify(const float* params, uint32_t n, uint32_t* deadFlag, uint32_t* donorFlag,
                             cudaStream_t s);

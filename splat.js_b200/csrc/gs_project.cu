@@ -305,6 +305,8 @@ __global__ void k_tile_ranges_finish(TileRangeArgs a, uint32_t totalTiles) {
   for (int u = 0; u < v; ++u) base += a.viewTotal[u];
   const uint2 r = a.ranges[gt];
   a.ranges[gt] = make_uint2(r.x + base, r.y + base);
+  const uint32_t b = tile_bucket(r), peers = __match_any_sync(__activemask(), b);
+  if ((threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&a.buckets[b], (uint32_t)__popc(peers));
 }
 
 // The live columns of one tile row of an item's rectangle.  tileLive(tx, ty)
@@ -368,9 +370,10 @@ __device__ __forceinline__ uint32_t block_bits(uint32_t b0, uint32_t b1, uint32_
 }
 
 // Entry expansion of the presorted items, in two passes over the same walk:
-// KEYS = false counts each item's entries, KEYS = true writes them at the
-// counts' exclusive scan -- key = global tile id, value = splat id, tiles of
-// an item in row order.  An entry is a tile of the item's rectangle that the
+// KEYS = false counts each item's entries and each block's total, KEYS = true
+// writes them at the counts' exclusive scan (the scanned block totals plus a
+// scan inside the block) -- key = global tile id, value = splat id, tiles of an
+// item in row order.  An entry is a tile of the item's rectangle that the
 // entry budget kept and, with culling on, that tileLive() accepts (a
 // single-tile rectangle is kept untested).
 //
@@ -381,23 +384,24 @@ __device__ __forceinline__ uint32_t block_bits(uint32_t b0, uint32_t b1, uint32_
 // then fills the rows' outputs 32 entries at a time, each lane finding its
 // row by a second binary search, so stores are coalesced.  Items of views
 // that dropped tiles to the budget are walked by their own lane (rare).
+constexpr uint32_t EXPAND_STAGE = 256;  // entries of a 32-row chunk that shared memory holds
 template <bool KEYS>
 __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
+  static_assert(EXPAND_BLOCK == 256, "one item a thread");
   __shared__ uint32_t s_run[256];  // entries of each item so far
-  const uint64_t items = (uint64_t)a.n * a.V;
+  __shared__ uint32_t s_sum[8];    // entries of each warp's items
+  __shared__ uint2 s_out[KEYS ? 8 : 1][KEYS ? EXPAND_STAGE : 1];  // a chunk's entries (key, value)
   // culled items carry the all-ones key, which the presort drops: its output
   // holds the live items only
   const uint64_t live = *a.liveItems;
   const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if ((uint64_t)blockIdx.x * blockDim.x >= live) {  // the whole block is culled items (uniform)
-    if (!KEYS && p < items) a.counts[p] = 0u;
-    return;
-  }
+  if ((uint64_t)blockIdx.x * blockDim.x >= live) return;  // the whole block is culled items (uniform)
   const int lane = threadIdx.x & 31;
   const int wbase = threadIdx.x & ~31;
   const uint32_t FULL = 0xFFFFFFFFu;
   const bool valid = p < live;
-  uint32_t v = 0, i = 0, x0 = 0, x1 = 0, y0 = 0, rr = 0, out = 0;
+  uint32_t v = 0, i = 0, x0 = 0, x1 = 0, y0 = 0, rr = 0, out = 0, count = 0;
+  uint32_t y1own = 0xFFFFFFFFu;
   bool test = false;
   float mx = 0.0f, my = 0.0f;
   float4 cq = make_float4(__int_as_float(0x7F800000), 0.0f, 0.0f, 0.0f);
@@ -424,7 +428,7 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
       mx = __uint_as_float(e0.z); my = __uint_as_float(e0.w);
       cq = make_float4(__uint_as_float(e1.x), __uint_as_float(e1.y), __uint_as_float(e1.z), 0.0f);
       slot = e1.w;
-      out = a.offsets[p];
+      count = a.counts[p];
     }
     if (r.x != 0xFFFFFFFFu) {
       v = slot / a.n;
@@ -433,31 +437,43 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
       x1 = r.y & 0xFFFFu;
       const uint32_t y1 = r.y >> 16;
       test = a.cull && !(x0 == x1 && y0 == y1);
-      if (a.viewDrops[v] == 0) {
-        rr = y1 - y0 + 1;
-      } else {
-        const DevCam& c = a.cams[v];
-        const uint8_t* dr = a.dropped + c.tileBase;
-        uint32_t o = out, cnt = 0;
-        for (uint32_t y = y0; y <= y1; ++y)
-          for (uint32_t x = x0; x <= x1; ++x) {
-            const uint32_t t = y * c.tilesX + x;
-            if (dr[t]) continue;
-            if (test && !tileLive(cq, mx, my, (int)x, (int)y, a.tile, c.W, c.H)) continue;
-            if (KEYS) {
-              if (o < a.capacity) {
-                a.keys[o] = c.tileBase + t;
-                a.vals[o] = i | (a.masks ? block_bits(band_columns(cq, mx, my, y * 16, x),
-                                                      band_columns(cq, mx, my, y * 16 + 8, x), 0u) : 0u);
-              }
-              else atomicOr(a.status, ST_ENTRY_OVERFLOW);
-              ++o;
-            }
-            ++cnt;
-          }
-        s_run[threadIdx.x] = cnt;
-      }
+      if (a.viewDrops[v] == 0) rr = y1 - y0 + 1;
+      else y1own = y1;
     }
+  }
+  if (KEYS) {  // the item's first entry: the block's start plus a scan of the counts before it
+    uint32_t inc = count;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(FULL, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) s_sum[threadIdx.x >> 5] = inc;
+    __syncthreads();
+    out = a.partials[blockIdx.x] + inc - count;
+    for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) out += s_sum[w];
+  }
+  if (y1own != 0xFFFFFFFFu) {  // a view with dropped tiles: the lane walks its own rectangle
+    const DevCam& c = a.cams[v];
+    const uint8_t* dr = a.dropped + c.tileBase;
+    uint32_t o = out, cnt = 0;
+    for (uint32_t y = y0; y <= y1own; ++y)
+      for (uint32_t x = x0; x <= x1; ++x) {
+        const uint32_t t = y * c.tilesX + x;
+        if (dr[t]) continue;
+        if (test && !tileLive(cq, mx, my, (int)x, (int)y, a.tile, c.W, c.H)) continue;
+        if (KEYS) {
+          if (o < a.capacity) {
+            a.keys[o] = c.tileBase + t;
+            a.vals[o] = i | (a.masks ? block_bits(band_columns(cq, mx, my, y * 16, x),
+                                                  band_columns(cq, mx, my, y * 16 + 8, x), 0u) : 0u);
+          }
+          else atomicOr(a.status, ST_ENTRY_OVERFLOW);
+          ++o;
+        }
+        ++cnt;
+      }
+    s_run[threadIdx.x] = cnt;
   }
   __syncwarp();
   // row offsets of the warp's items (inclusive scan of rr)
@@ -467,6 +483,9 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
     const uint32_t y = __shfl_up_sync(FULL, rEnd, o);
     if (lane >= o) rEnd += y;
   }
+  // without items of views that dropped tiles between them, the rows' entries
+  // follow one another in the output
+  const bool dense = !__any_sync(FULL, y1own != 0xFFFFFFFFu);
   const uint32_t rBase = rEnd - rr;
   const uint32_t R = __shfl_sync(FULL, rEnd, 31);
   for (uint32_t base = 0; base < R; base += 32) {
@@ -522,6 +541,25 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
       const uint32_t oi = __shfl_sync(FULL, i, lo);
       const uint32_t tileBase = a.cams[ov].tileBase, tilesX = (uint32_t)a.cams[ov].tilesX;
       const uint32_t rowKey = tileBase + ty * tilesX + ca;  // key of the run's first tile
+      // Usual chunks go through shared memory: each lane writes its row's run
+      // there, and the warp copies the chunk out coalesced.  (The search below,
+      // 32 entries at a time, took 461 us for 30M entries with block bits.)
+      const uint32_t chunk = __shfl_sync(FULL, inc, 31);  // entries of the 32 rows
+      const uint32_t chunkOut = __shfl_sync(FULL, oout + prior, 0);  // where they start
+      if (dense && chunk <= EXPAND_STAGE) {
+        uint2* st = s_out[threadIdx.x >> 5];
+        uint32_t at = inc - cnt;  // rows follow one another in output order
+        for (uint32_t j = 0; j < cnt; ++j, ++at)
+          st[at] = make_uint2(rowKey + j, oi | (a.masks ? block_bits(band0, band1, 2u * j) : 0u));
+        __syncwarp();
+        for (uint32_t k = (uint32_t)lane; k < chunk; k += 32) {
+          const uint2 kv = st[k];
+          const uint64_t e = (uint64_t)chunkOut + k;
+          if (e < a.capacity) { a.keys[e] = kv.x; a.vals[e] = kv.y; }
+          else atomicOr(a.status, ST_ENTRY_OVERFLOW);
+        }
+        __syncwarp();
+      } else {
       // the chunk's rows in output order: rowOut is non-decreasing over lanes with entries
       const uint32_t firstOut = __reduce_min_sync(FULL, cnt ? rowOut : 0xFFFFFFFFu);
       uint32_t lastEnd = __reduce_max_sync(FULL, cnt ? rowOut + cnt : 0u);
@@ -556,6 +594,7 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
           else atomicOr(a.status, ST_ENTRY_OVERFLOW);
         }
       }
+      }
     }
     uint32_t gsum = 0;
     if (inRange) gsum = __reduce_add_sync(peers, cnt);  // the lanes of one item call it together
@@ -563,7 +602,19 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
     if (inRange && lane == lead) s_run[wbase + lo] = prior + gsum;
     __syncwarp();
   }
-  if (!KEYS && p < items) a.counts[p] = valid ? s_run[threadIdx.x] : 0u;
+  if (!KEYS) {
+    const uint32_t cnt = valid ? s_run[threadIdx.x] : 0u;
+    if (valid) a.counts[p] = cnt;
+    const uint32_t sum = __reduce_add_sync(FULL, cnt);
+    if (lane == 0) s_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t all = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) all += s_sum[w];
+      a.partials[blockIdx.x] = all;
+    }
+  }
 }
 
 // Per-tile ranges from the sorted entry keys (culled lists): tile gt spans
@@ -579,12 +630,52 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t* keys, uint32
   return lo;
 }
 
+// Up to WARP_SEARCH_TILES tiles a warp searches for one bound, 33-ary: each
+// lane probes one pivot and a ballot says how many of them hold smaller keys,
+// so 30M entries take six dependent loads.  With more tiles the chip is full
+// anyway and a thread per bound does less work: 25 dependent loads, but a
+// thirty-second of the instructions.  (One thread per tile searching for both
+// its bounds took 6.3 us at 450 tiles and 21 us at 65k; the warps take 3 us
+// at 450 and, searching for both bounds, 39 us at 65k.)  A block's last bound is
+// only the end of the tile before it.  Counts the tiles per work-order bucket,
+// with one atomic per bucket per warp.
+constexpr uint32_t WARP_SEARCH_TILES = 8192;
+template <bool WARP>
 __global__ void __launch_bounds__(256) k_ranges_from_keys(const uint32_t* keys, const uint32_t* nItems,
-                                                          uint32_t totalTiles, uint2* ranges) {
-  const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gt >= totalTiles) return;
+                                                          uint32_t totalTiles, uint2* ranges, uint32_t* buckets) {
+  constexpr uint32_t PER = WARP ? 8u : 256u;  // bounds per block
+  __shared__ uint32_t s_bound[PER];
+  const uint32_t FULL = 0xFFFFFFFFu, lane = threadIdx.x & 31u;
+  const uint32_t own = WARP ? threadIdx.x >> 5 : threadIdx.x;
+  const uint32_t gt = blockIdx.x * (PER - 1u) + own;  // first key >= gt
   const uint32_t E = *nItems;
-  ranges[gt] = make_uint2(lower_bound_u32(keys, E, gt), lower_bound_u32(keys, E, gt + 1));
+  if (WARP) {
+    uint32_t lo = 0, hi = gt <= totalTiles ? E : 0u;
+    while (lo < hi) {
+      const uint32_t step = (hi - lo) / 33u + 1u;
+      const uint64_t p = (uint64_t)lo + (uint64_t)step * (lane + 1u) - 1u;
+      const bool below = p < hi && keys[p] < gt;
+      const uint32_t c = (uint32_t)__popc(__ballot_sync(FULL, below));
+      // pivots up to c hold smaller keys, pivot c + 1 (if it lies in the range) does not
+      const uint64_t next = (uint64_t)lo + (uint64_t)step * (c + 1u) - 1u;
+      if (next < hi && c < 32u) hi = (uint32_t)next;
+      lo += step * c;
+    }
+    if (lane == 0) s_bound[own] = lo;
+  } else {
+    s_bound[own] = gt <= totalTiles ? lower_bound_u32(keys, E, gt) : 0u;
+  }
+  __syncthreads();
+  if (WARP && threadIdx.x >= 32u) return;
+  const uint32_t k = threadIdx.x, tile = blockIdx.x * (PER - 1u) + k;
+  uint32_t b = 64u;
+  if (k < PER - 1u && tile < totalTiles) {
+    const uint2 r = make_uint2(s_bound[k], s_bound[k + 1]);
+    ranges[tile] = r;
+    b = tile_bucket(r);
+  }
+  const uint32_t peers = __match_any_sync(FULL, b);
+  if (b < 64u && lane == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&buckets[b], (uint32_t)__popc(peers));
 }
 
 void launch_step_begin(const StepBeginArgs& a, cudaStream_t s) {
@@ -615,8 +706,12 @@ void launch_expand(const ExpandArgs& a, bool keys, cudaStream_t s) {
   else k_expand<false><<<grid, 256, 0, s>>>(a);
 }
 void launch_ranges_from_keys(const uint32_t* keys, const uint32_t* nItems, uint32_t totalTiles, uint2* ranges,
-                             cudaStream_t s) {
-  if (totalTiles) k_ranges_from_keys<<<(totalTiles + 255) / 256, 256, 0, s>>>(keys, nItems, totalTiles, ranges);
+                             uint32_t* buckets, cudaStream_t s) {
+  if (totalTiles == 0) return;
+  if (totalTiles <= WARP_SEARCH_TILES)
+    k_ranges_from_keys<true><<<(totalTiles + 6) / 7, 256, 0, s>>>(keys, nItems, totalTiles, ranges, buckets);
+  else
+    k_ranges_from_keys<false><<<(totalTiles + 254) / 255, 256, 0, s>>>(keys, nItems, totalTiles, ranges, buckets);
 }
 
 }  // namespace gs

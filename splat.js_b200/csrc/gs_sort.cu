@@ -75,30 +75,52 @@ __global__ void __launch_bounds__(1024) k_scan_reduce(const uint32_t* in, uint64
   if (threadIdx.x == 0) partials[blockIdx.x] = tot;
 }
 
-// single block: exclusive scan of the block sums, total to *total
-__global__ void __launch_bounds__(1024) k_scan_partials(uint32_t* partials, uint32_t nb, uint32_t* total) {
+// single block: exclusive scan of nb block sums in place, total to *total
+template <int ITEMS>
+__device__ __forceinline__ void scan_in_place(uint32_t* partials, uint32_t nb, uint32_t* total) {
   __shared__ uint32_t s_warp[33];
-  __shared__ uint32_t s_carry;
-  if (threadIdx.x == 0) s_carry = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < nb; base += 1024 * SCAN_ITEMS) {
-    const uint32_t i0 = base + threadIdx.x * SCAN_ITEMS;
-    uint32_t v[SCAN_ITEMS];
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < nb; base += 1024 * ITEMS) {
+    const uint32_t i0 = base + threadIdx.x * ITEMS;
+    uint32_t v[ITEMS];
     uint32_t s = 0;
 #pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) { v[k] = (i0 + k < nb) ? partials[i0 + k] : 0u; s += v[k]; }
-    uint32_t tot;
-    uint32_t ex = block_exclusive_scan_1024(s, s_warp, &tot) + s_carry;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; ++k) {
-      if (i0 + k < nb) partials[i0 + k] = ex;
-      ex += v[k];
+    for (int k = 0; k < ITEMS; k += 4) {  // the array is padded to a multiple of 4
+      const uint4 q = i0 + k < nb ? *reinterpret_cast<const uint4*>(partials + i0 + k) : make_uint4(0u, 0u, 0u, 0u);
+      v[k] = q.x;
+      v[k + 1] = i0 + k + 1 < nb ? q.y : 0u;
+      v[k + 2] = i0 + k + 2 < nb ? q.z : 0u;
+      v[k + 3] = i0 + k + 3 < nb ? q.w : 0u;
+      s += v[k] + v[k + 1] + v[k + 2] + v[k + 3];
     }
-    __syncthreads();
-    if (threadIdx.x == 0) s_carry += tot;
-    __syncthreads();
+    uint32_t tot;
+    uint32_t ex = block_exclusive_scan_1024(s, s_warp, &tot) + carry;
+#pragma unroll
+    for (int k = 0; k < ITEMS; k += 4) {
+      const uint4 q = make_uint4(ex, ex + v[k], ex + v[k] + v[k + 1], ex + v[k] + v[k + 1] + v[k + 2]);
+      if (i0 + k < nb) *reinterpret_cast<uint4*>(partials + i0 + k) = q;
+      ex = q.w + v[k + 3];
+    }
+    carry += tot;
   }
-  if (threadIdx.x == 0) *total = s_carry;
+  if (threadIdx.x == 0) *total = carry;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_partials(uint32_t* partials, uint32_t nb, uint32_t* total) {
+  scan_in_place<SCAN_ITEMS>(partials, nb, total);
+}
+
+// the same over the blocks of perBlock of *nItems items
+__global__ void __launch_bounds__(1024) k_scan_blocks(uint32_t* partials, const uint32_t* nItems, uint32_t perBlock,
+                                                      uint32_t* total) {
+  const uint32_t nb = (*nItems + perBlock - 1) / perBlock;
+  if (nb <= 1024 * SCAN_ITEMS) scan_in_place<SCAN_ITEMS>(partials, nb, total);
+  else scan_in_place<16>(partials, nb, total);
+}
+
+void launch_scan_blocks(uint32_t* partials, const uint32_t* nItems, uint32_t perBlock, uint32_t* total,
+                        cudaStream_t s) {
+  k_scan_blocks<<<1, 1024, 0, s>>>(partials, nItems, perBlock, total);
 }
 
 __global__ void __launch_bounds__(1024) k_scan_down(const uint32_t* in, uint64_t N, const uint32_t* partials,

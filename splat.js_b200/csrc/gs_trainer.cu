@@ -79,7 +79,7 @@ struct gs_trainer {
   float *params = nullptr, *m = nullptr, *v = nullptr, *sh = nullptr, *shM = nullptr, *shV = nullptr;
   RenderRec* recs = nullptr;
   uint2* rect = nullptr;
-  uint32_t *counts = nullptr, *offsets = nullptr;
+  uint32_t* counts = nullptr;
   float4* cullRecs = nullptr;
   uint4* itemRecs = nullptr;
   float* viewGrad = nullptr;
@@ -422,7 +422,6 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
   GS_AL(h->viewTotal, (size_t)MAXB);
   GS_AL(h->rect, (size_t)B * cap);
   GS_AL(h->counts, (size_t)B * cap);
-  GS_AL(h->offsets, (size_t)B * cap);
   GS_AL(h->cullRecs, (size_t)B * cap);
   GS_AL(h->itemRecs, (size_t)B * cap * 2);
   GS_AL(h->itemSrc, (size_t)B * cap * 2);
@@ -442,7 +441,7 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
   GS_AL(h->vals[1], h->capacity);
   GS_AL(h->small, (size_t)4096);
   GS_AL(h->lbStatus, (size_t)(std::max<uint64_t>(h->capacity, (uint64_t)B * cap) / SORT_BLOCK_ENTRIES + 2) * 256);
-  GS_AL(h->scanPartials, (size_t)scan_partials_needed((uint64_t)B * cap) + 1);
+  GS_AL(h->scanPartials, (size_t)B * cap / EXPAND_BLOCK + 4);  // padded: scanned four words at a time
   GS_AL(h->outImg, (size_t)B * h->maxPix);
   GS_AL(h->finalT, (size_t)B * h->maxPix);
   GS_AL(h->endIdx, (size_t)B * h->maxPix);
@@ -667,6 +666,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   const bool masks = block_masks(sh.tile, sh.n);
   uint32_t* nItems = h->small + 2061;
   uint32_t* liveItems = h->small + 2150;
+  uint32_t* buckets = h->small + 2080;  // 33 sizes and 33 cursors of the work order
   {
     StepBeginArgs ba{};
     ba.ring = reinterpret_cast<const uint32_t*>(h->hRing);
@@ -720,6 +720,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   ta.stats = h->stats;
   ta.entriesCap = h->entriesCap;
   ta.totalEntries = totalEntries;
+  ta.buckets = buckets;
   ta.ranges = cull ? nullptr : h->ranges;  // culled lists take their ranges from the sorted keys
   if (fork) {
     cudaEventRecord(h->forkEv, s);
@@ -771,14 +772,14 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   ea.cull = cull ? 1 : 0;
   ea.masks = masks ? 1 : 0;
   ea.counts = h->counts;
-  ea.offsets = h->offsets;
+  ea.partials = h->scanPartials;
   ea.keys = h->keys[0];
   ea.vals = h->vals[0];
   ea.capacity = h->capacity;
   ea.status = statusWord;
   launch_expand(ea, false, s);
   // culled lists: the entry total is the counts' sum, not the budgeted tile sum
-  launch_exclusive_scan(h->counts, items, h->offsets, h->scanPartials, cull ? totalEntries : scanTotal, s);
+  launch_scan_blocks(h->scanPartials, liveItems, EXPAND_BLOCK, cull ? totalEntries : scanTotal, s);
   launch_expand(ea, true, s);
 
   // stable sort of the entries by global tile id: at most 4 passes, with
@@ -802,16 +803,16 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   launch_radix_sort(ra, s);
   h->lastPasses = passes;
   h->lastMasks = masks;
-  if (cull) launch_ranges_from_keys(h->keys[passes & 1], totalEntries, totalTiles, h->ranges, s);
+  if (cull) launch_ranges_from_keys(h->keys[passes & 1], totalEntries, totalTiles, h->ranges, buckets, s);
   // kernels: begin, project, tile counts [+ finish], presort (histogram + passes),
-  // entry counts, 3 scan kernels, entry keys, tile sort (histogram +
-  // passes), [ranges from keys], [work order: 3], raster, [visible lists, chain per view, sum + Adam]
-  h->lastLaunches = (cull ? 3u : 4u) + 1u + (uint32_t)pr.passes + 1u + 3u + 1u + 1u + (uint32_t)passes + (cull ? 1u : 0u) +
-                    (h->o.persistent ? 3u : 0u) + 1u + (sh.chain ? 3u : 0u);
+  // entry counts, scan, entry keys, tile sort (histogram + passes),
+  // [ranges from keys], [work order], raster, [visible lists, chain per view, sum + Adam]
+  h->lastLaunches = (cull ? 3u : 4u) + 1u + (uint32_t)pr.passes + 1u + 1u + 1u + 1u + (uint32_t)passes + (cull ? 1u : 0u) +
+                    (h->o.persistent ? 1u : 0u) + 1u + (sh.chain ? 3u : 0u);
   const uint32_t* sortedIds = h->vals[passes & 1];
 
   const bool persistent = h->o.persistent != 0;
-  if (persistent) launch_work_order(h->ranges, totalTiles, h->workOrder, h->small + 2080, s);  // [2080, 2146)
+  if (persistent) launch_work_place(h->ranges, totalTiles, buckets, buckets + 33, h->workOrder, s);
   if (h->profiling) cudaEventRecord(ph[2], s);
   RasterArgs rr{};
   rr.cams = dcams;
@@ -1474,7 +1475,7 @@ int gs_refine(gs_trainer* h, gs_rng_fn rng, void* ctx, gs_refine_result* out) {
     GS_AL(h->rf.donorList, cap);
     GS_AL(h->rf.splitSeq, cap);
     GS_AL(h->rf.plan, cap);
-    GS_AL(h->rf.partials, (size_t)scan_partials_needed(cap) + 1);
+    GS_AL(h->rf.partials, (size_t)scan_partials_needed(cap) + 4);
     GS_AL(h->rf.counts, (size_t)4);
 #undef GS_AL
   }
