@@ -21,14 +21,14 @@ struct CamGrad7 {
 };
 
 // chain for one visible splat in one view; gp = decoded screen-space grads
-// shp: the splat's SH coefficients in global memory (read through the
-// cache).  The SH coefficient gradients are dRGB[c] * Y[k] for k < aK: the
+// shp: the splat's SH row in shared memory (ShRows).  The SH coefficient gradients are dRGB[c] * Y[k] for k < aK: the
 // gated dRGB, Y and aK are returned instead of the 3K products.
 template <int DEG>
 __device__ __forceinline__ void chainOne(const DevCam& c, const float* P, const Geom& g, float gp[10],
                                          const float* shp, float anisoReg, float gF[16], float dRGBo[3],
                                          float Yo[15], float vdo[3], int& aKo, CamGrad7& cg) {
-  constexpr int K = DEG > 0 ? (DEG + 1) * (DEG + 1) - 1 : 0;
+  using Rows = ShRows<DEG>;
+  constexpr int K = Rows::K;
   const float f = c.f, z = g.pc[2], iz = 1.0f / z;
   // conic -> dilated 2D covariance (shaders.js:758-777)
   const float ad = g.va + 0.3f, cd = g.vc + 0.3f;
@@ -185,23 +185,35 @@ __device__ __forceinline__ void chainOne(const DevCam& c, const float* P, const 
     aKo = aK;
     float col[3] = {sCol[0], sCol[1], sCol[2]};
 #pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (k < aK) {
-        col[0] = col[0] + __ldg(shp + k) * Yo[k];
-        col[1] = col[1] + __ldg(shp + K + k) * Yo[k];
-        col[2] = col[2] + __ldg(shp + 2 * K + k) * Yo[k];
-      }
+    for (int k = 0; k < K; k += Rows::GROUP)
+      if (k < aK)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          float c3[Rows::GROUP];
+          Rows::load(shp, j, k, c3);
+#pragma unroll
+          for (int q = 0; q < Rows::GROUP; ++q)
+            if (k + q < aK) col[j] = col[j] + c3[q] * Yo[k + q];
+        }
 #pragma unroll
     for (int j = 0; j < 3; ++j) dRGB[j] = dRGB[j] * (col[j] > 0.0f ? 1.0f : 0.0f);
     float gv[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int k = 0; k < K; ++k)
+    for (int k = 0; k < K; k += Rows::GROUP)
       if (k < aK) {
-        const float wk = dRGB[0] * __ldg(shp + k) + dRGB[1] * __ldg(shp + K + k) + dRGB[2] * __ldg(shp + 2 * K + k);
-        float D[3];
-        shBasisGradK<DEG>(k, vd, D);
+        float c0[Rows::GROUP], c1[Rows::GROUP], c2[Rows::GROUP];
+        Rows::load(shp, 0, k, c0);
+        Rows::load(shp, 1, k, c1);
+        Rows::load(shp, 2, k, c2);
 #pragma unroll
-        for (int j = 0; j < 3; ++j) gv[j] = gv[j] + wk * D[j];
+        for (int q = 0; q < Rows::GROUP; ++q)
+          if (k + q < aK) {
+            const float wk = dRGB[0] * c0[q] + dRGB[1] * c1[q] + dRGB[2] * c2[q];
+            float D[3];
+            shBasisGradK<DEG>(k + q, vd, D);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) gv[j] = gv[j] + wk * D[j];
+          }
       }
     const float vg = dot3(vd, gv);
 #pragma unroll
@@ -290,7 +302,8 @@ __global__ void __launch_bounds__(256) k_visible_list(ChainArgs a, uint32_t bloc
 // summed per warp in fixed point (order-independent) with one atomic each.
 template <int DEG>
 __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainArgs a) {
-  constexpr int K = DEG > 0 ? (DEG + 1) * (DEG + 1) - 1 : 0;
+  using Rows = ShRows<DEG>;
+  constexpr int K = Rows::K;
   const uint32_t sb = blockIdx.x / (uint32_t)a.V;
   const int v = (int)(blockIdx.x - sb * (uint32_t)a.V);
   const uint32_t pos = sb * blockDim.x + threadIdx.x;
@@ -304,6 +317,21 @@ __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainAr
   // before the barrier that publishes it
   __shared__ DevCam s_cam;
   copy_cams(&s_cam, a.cams + v, 1);
+  // each warp copies the SH rows of its own items, whole rows by neighbouring lanes
+  __shared__ __align__(16) float s_sh[K > 0 ? 128 * Rows::PITCH : 4];
+  float* const warpRows = s_sh + (K > 0 ? (threadIdx.x & ~31u) * Rows::PITCH : 0);
+  if (K > 0) {
+    constexpr int PART = DEG == 2 ? 4 : 1, PARTS = K > 0 ? Rows::WORDS / PART : 1;  // words per copy, copies per row
+#pragma unroll 5
+    for (int j = 0; j < PARTS; ++j) {
+      const int e = lane + 32 * j, row = e / PARTS, col = (e - row * PARTS) * PART;
+      const uint32_t id = __shfl_sync(0xFFFFFFFFu, i, row);
+      const float* src = a.sh + (size_t)id * Rows::WORDS + col;
+      if (PART == 4) cp_async16(warpRows + row * Rows::PITCH + col, src);
+      else cp_async4(warpRows + row * Rows::PITCH + col, src);
+    }
+    cp_async_commit();
+  }
   const size_t slot = (size_t)v * a.n + i;
   int4 q0 = make_int4(0, 0, 0, 0), q1 = q0, q2 = q0;
   float P[16];
@@ -317,6 +345,7 @@ __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainAr
       P[4 * k] = t.x; P[4 * k + 1] = t.y; P[4 * k + 2] = t.z; P[4 * k + 3] = t.w;
     }
   }
+  cp_async_wait<0>();
   __syncthreads();
   const DevCam& c = s_cam;
   CamGrad7 cg = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, 0.0f};
@@ -343,7 +372,7 @@ __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainAr
         const float lmax = cmid + sqrtf(fmaxf(cmid * cmid - (cva * cvc - g.vb * g.vb), 0.0f));
         const float cden = 1.0f + lmax;
         gp[2] = gp[2] * cden; gp[3] = gp[3] * cden; gp[4] = gp[4] * cden;
-        const float* shp = K > 0 ? a.sh + (size_t)i * 3 * K : nullptr;
+        const float* shp = warpRows + (K > 0 ? lane * Rows::PITCH : 0);
         chainOne<DEG>(c, P, g, gp, shp, a.anisoReg, gF, dRGB, Y, vd, aK, cg);
       }
       float4* o = reinterpret_cast<float4*>(a.viewGrad + slot * VIEWGRAD_STRIDE);

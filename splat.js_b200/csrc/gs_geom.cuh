@@ -131,6 +131,30 @@ __device__ __forceinline__ void shBasis(const float v[3], float Y[15]) {
   }
 }
 
+// SH rows staged in shared memory.  Read from global memory, each of a splat's
+// 3K coefficients is a load whose 32 lanes lie a whole row (36-180 B) apart, a
+// wavefront per lane; one wavefront per clock per SM was what bounded the
+// projection and the chain.  Rows are copied coalesced (cp.async) and read at a
+// stride without bank conflicts: 9 and 45 words are odd; the 24 words of
+// degree 2 are padded to 28 and read four at a time, so eight lanes cover the
+// 32 banks.
+template <int DEG>
+struct ShRows {
+  static constexpr int K = DEG > 0 ? (DEG + 1) * (DEG + 1) - 1 : 0;
+  static constexpr int WORDS = 3 * K;                              // of a row
+  static constexpr int PITCH = DEG == 2 ? 28 : (K > 0 ? WORDS : 1);  // words between rows
+  static constexpr int GROUP = DEG == 2 ? 4 : 1;                   // coefficients read together
+  // coefficients [k, k + GROUP) of channel ch
+  static __device__ __forceinline__ void load(const float* row, int ch, int k, float v[GROUP]) {
+    if constexpr (DEG == 2) {
+      const float4 q = *reinterpret_cast<const float4*>(row + ch * K + k);
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+      v[0] = row[ch * K + k];
+    }
+  }
+};
+
 template <int DEG>
 __device__ __forceinline__ void shBasisGrad(const float v[3], float D[15][3]) {
   const float x = v[0], y = v[1], z = v[2];

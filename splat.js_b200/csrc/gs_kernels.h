@@ -17,8 +17,9 @@ constexpr uint32_t GRID_COPIES = 4;
 
 // First kernel of a pass (k_step_begin).
 struct StepBeginArgs {
-  const uint32_t* ring;    // pinned host memory: `slots` parameter records of `words` words
-  uint32_t slots, words;
+  const uint32_t* ring;    // pinned host memory: `slots` parameter records `stride` words apart
+  uint32_t slots, stride;
+  uint32_t words;          // words of the record that the pass needs
   uint32_t* seq;           // passes run so far: this one takes slot seq % slots
   uint32_t* params;        // device copy of the record
   uint32_t* nItems;        // presort items of the pass, set to `items`
@@ -101,6 +102,13 @@ struct RadixHistArgs {
 #define GS_SORT_ITEMS 16  // keys per thread of a onesweep block (256 threads)
 #endif
 constexpr int SORT_BLOCK_ENTRIES = 256 * GS_SORT_ITEMS;  // entries one onesweep block ranks
+constexpr uint32_t RS_SMALL = 256u * 1024u;              // up to here blocks of a quarter of that
+// look-back words (per digit) that sorts of up to N entries use
+constexpr uint64_t sort_status_blocks(uint64_t N) {
+  const uint64_t big = (N + SORT_BLOCK_ENTRIES - 1) / SORT_BLOCK_ENTRIES;
+  const uint64_t few = (N < RS_SMALL ? N : RS_SMALL), small = (few + SORT_BLOCK_ENTRIES / 4 - 1) / (SORT_BLOCK_ENTRIES / 4);
+  return big > small ? big : small;
+}
 
 struct OnesweepArgs {
   const void* keysIn;
@@ -115,6 +123,7 @@ struct OnesweepArgs {
   const uint32_t* epoch;
   int pass;
   uint32_t spinLimit;       // look-back spins before the block gives up and flags a timeout
+  int smallBlocks;          // 1: few entries are sorted in blocks of a quarter of the size
   int dropAllOnes;          // all-ones keys leave the sort (output compacted to the kept keys);
                             // selects the kernel instantiation that drops them
 };

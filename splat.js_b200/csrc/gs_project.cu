@@ -35,30 +35,53 @@ namespace gs {
 // round trip of the record (2.2 KB).
 __global__ void __launch_bounds__(256) k_step_begin(StepBeginArgs a) {
   if (blockIdx.x == 0) {
-    const uint32_t* src = a.ring + (size_t)(*a.seq % a.slots) * a.words;
-    for (uint32_t k = threadIdx.x; k < a.words; k += blockDim.x) {
-      uint32_t w;  // written by the host before the launch: not from a cache
-      asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(w) : "l"(src + k));
-      a.params[k] = w;
+    const uint32_t* src = a.ring + (size_t)(*a.seq % a.slots) * a.stride;
+    uint32_t w[3];  // a record has at most 3 x 256 words: all loads in flight together
+#pragma unroll
+    for (uint32_t r = 0; r < 3; ++r) {
+      const uint32_t k = threadIdx.x + 256u * r;
+      // written by the host before the launch: not from a cache
+      if (k < a.words) asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(w[r]) : "l"(src + k));
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < 3; ++r) {
+      const uint32_t k = threadIdx.x + 256u * r;
+      if (k < a.words) a.params[k] = w[r];
     }
     __syncthreads();
     if (threadIdx.x == 0) {
       *a.seq += 1u;
       *a.nItems = a.items;
     }
-  }
-  const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  } else {
+    const uint32_t at = (blockIdx.x - 1u) * blockDim.x + threadIdx.x, stride = (gridDim.x - 1u) * blockDim.x;
 #pragma unroll
-  for (int r = 0; r < 3; ++r)
-    for (uint32_t k = at; k < a.count[r]; k += stride) a.clear[r][k] = 0u;
+    for (int r = 0; r < 3; ++r)
+      for (uint32_t k = at; k < a.count[r]; k += stride) a.clear[r][k] = 0u;
+  }
 }
 
 // One thread per splat, looping over the batch's views: parameters and SH
 // coefficients are read once per step.
+constexpr int PROJECT_THREADS = 128;
 template <int DEG>
-__global__ void __launch_bounds__(256, 4) k_project(ProjectArgs a) {  // 4 blocks/SM: 64 registers
-  constexpr int K = DEG > 0 ? (DEG + 1) * (DEG + 1) - 1 : 0;
+__global__ void __launch_bounds__(PROJECT_THREADS, 8) k_project(ProjectArgs a) {  // 8 blocks/SM: 64 registers
+  using Rows = ShRows<DEG>;
+  constexpr int K = Rows::K;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ __align__(16) float s_sh[K > 0 ? PROJECT_THREADS * Rows::PITCH : 4];
+  if (K > 0) {  // the block's SH rows, contiguous in global memory and 16-byte aligned at its first
+    const uint32_t i0 = blockIdx.x * PROJECT_THREADS;
+    const uint32_t words = min(a.n - i0, (uint32_t)PROJECT_THREADS) * Rows::WORDS;
+    const float* src = a.sh + (size_t)i0 * Rows::WORDS;
+    for (uint32_t c = threadIdx.x; 4 * c < words; c += PROJECT_THREADS) {
+      // degree 2: a row is six 16-byte chunks; else rows lie as in global memory
+      const uint32_t at = DEG == 2 ? (c / 6u) * Rows::PITCH + (c % 6u) * 4u : 4u * c;
+      if (4 * c + 4 <= words) cp_async16(s_sh + at, src + 4 * c);
+      else for (uint32_t w = 4 * c; w < words; ++w) cp_async4(s_sh + at + (w - 4 * c), src + w);
+    }
+    cp_async_commit();
+  }
   // the batch's cameras in shared memory (read once per block); each thread
   // issues its parameter loads before the barrier that publishes them
   __shared__ DevCam s_cams[MAX_VIEWS];
@@ -72,9 +95,10 @@ __global__ void __launch_bounds__(256, 4) k_project(ProjectArgs a) {  // 4 block
       P[4 * k] = t.x; P[4 * k + 1] = t.y; P[4 * k + 2] = t.z; P[4 * k + 3] = t.w;
     }
   }
+  cp_async_wait<0>();
   __syncthreads();
   if (i >= a.n) return;
-  const float* shp = K > 0 ? a.sh + (size_t)i * 3 * K : nullptr;
+  const float* shp = s_sh + (K > 0 ? threadIdx.x * Rows::PITCH : 0);
   const float sig0 = sigm(P[10]), sig1 = sigm(P[11]), sig2 = sigm(P[12]);
   const float opa = sigm(P[13]);
 
@@ -113,13 +137,16 @@ __global__ void __launch_bounds__(256, 4) k_project(ProjectArgs a) {  // 4 block
       shBasis<DEG>(vd, Y);
       const int aK = shActiveK(c, K);
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        if (k < aK) {
-          col[0] = col[0] + __ldg(shp + k) * Y[k];
-          col[1] = col[1] + __ldg(shp + K + k) * Y[k];
-          col[2] = col[2] + __ldg(shp + 2 * K + k) * Y[k];
-        }
-      }
+      for (int k = 0; k < K; k += Rows::GROUP)
+        if (k < aK)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            float c3[Rows::GROUP];
+            Rows::load(shp, j, k, c3);
+#pragma unroll
+            for (int q = 0; q < Rows::GROUP; ++q)
+              if (k + q < aK) col[j] = col[j] + c3[q] * Y[k + q];
+          }
 #pragma unroll
       for (int j = 0; j < 3; ++j) col[j] = fmaxf(col[j], 0.0f);
     }
@@ -352,10 +379,10 @@ __device__ __forceinline__ uint32_t band_columns(const float4 cq, float mx, floa
   float xl, xr;
   if (!bandIntervalMask(cq, Y0, Y0 + 7.0f, xl, xr)) return 1u;
   const float sl = 4.0e-6f * (fabsf(mx) + fmaxf(fabsf(xl), fabsf(xr)) + 8.0f);
-  const float base = 2.0f * (float)ca;
-  const float l = clampf(ceilf(((xl + mx) - 7.5f - sl) * 0.125f) - base, 0.0f, 65535.0f);
-  const float r = clampf(floorf(((xr + mx) - 0.5f + sl) * 0.125f) - base, -1.0f, 65535.0f);
-  if (r < 0.0f) return 1u;
+  const int base = 2 * (int)ca;
+  const int l = min(max(__float2int_ru(fminf(((xl + mx) - 7.5f - sl) * 0.125f, 1.0e9f)) - base, 0), 65535);
+  const int r = min(__float2int_rd(fmaxf(((xr + mx) - 0.5f + sl) * 0.125f, -1.0e9f)) - base, 65535);
+  if (r < 0) return 1u;
   return (uint32_t)l | ((uint32_t)r << 16);
 }
 // block bits of a tile whose left block column is col: bands b0 (rows 0-7), b1
@@ -681,17 +708,17 @@ __global__ void __launch_bounds__(256) k_ranges_from_keys(const uint32_t* keys, 
 void launch_step_begin(const StepBeginArgs& a, cudaStream_t s) {
   uint32_t words = 0;
   for (int r = 0; r < 3; ++r) words = a.count[r] > words ? a.count[r] : words;
-  const unsigned blocks = (words + 1023) / 1024;  // four words a thread
-  k_step_begin<<<blocks < 296 ? (blocks ? blocks : 1) : 296, 256, 0, s>>>(a);
+  const unsigned blocks = (words + 1023) / 1024;  // clearing, four words a thread
+  k_step_begin<<<1 + (blocks < 296 ? (blocks ? blocks : 1) : 296), 256, 0, s>>>(a);
 }
 void launch_project(const ProjectArgs& a, int deg, cudaStream_t s) {
-  const unsigned grid = (a.n + 255) / 256;
+  const unsigned grid = (a.n + PROJECT_THREADS - 1) / PROJECT_THREADS;
   if (grid == 0) return;
   switch (deg) {
-    case 0: k_project<0><<<grid, 256, 0, s>>>(a); break;
-    case 1: k_project<1><<<grid, 256, 0, s>>>(a); break;
-    case 2: k_project<2><<<grid, 256, 0, s>>>(a); break;
-    default: k_project<3><<<grid, 256, 0, s>>>(a); break;
+    case 0: k_project<0><<<grid, PROJECT_THREADS, 0, s>>>(a); break;
+    case 1: k_project<1><<<grid, PROJECT_THREADS, 0, s>>>(a); break;
+    case 2: k_project<2><<<grid, PROJECT_THREADS, 0, s>>>(a); break;
+    default: k_project<3><<<grid, PROJECT_THREADS, 0, s>>>(a); break;
   }
 }
 void launch_tile_ranges(const TileRangeArgs& a, uint32_t totalTiles, cudaStream_t s) {

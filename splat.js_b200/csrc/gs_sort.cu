@@ -218,25 +218,36 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // replace the eight votes and their bit tests; lanes with equal digits hit
 // the same word, so it pays where a warp's digits are spread (tile ids) and
 // not where most of them are equal (the top bytes of depths).
-template <typename KT, bool DROP = false, bool ORM = false>
-#ifndef GS_SORT_MIN_BLOCKS
-#define GS_SORT_MIN_BLOCKS 3  // resident blocks per SM the register allocation must allow
-#endif
-__global__ void __launch_bounds__(RS_THREADS, GS_SORT_MIN_BLOCKS) k_onesweep(OnesweepArgs a) {
+template <bool ORM>
+struct OnesweepShared {
+  uint32_t whist[RS_WARPS][256];
+  uint32_t count[256];  // this block's count per digit
+  uint32_t run[256];    // the same, kept for the look-back
+  uint32_t local[256];  // exclusive prefix of count over digits
+  uint32_t gbase[256];  // global start of this block's run per digit
+  uint32_t dbase[256];  // exclusive scan of the pass histogram
+  uint32_t warp[33];
+  uint32_t tile;
+  uint32_t match[ORM ? RS_WARPS : 1][256];  // OR form: per warp, lanes holding each digit
+};
+// RS_ITEMS: entries per thread of a block.
+template <typename KT, bool DROP, bool ORM, int RS_ITEMS>
+__device__ __forceinline__ void onesweep_body(const OnesweepArgs& a, OnesweepShared<ORM>& sh) {
+  constexpr int RS_TILE = RS_THREADS * RS_ITEMS;  // entries per block
   extern __shared__ __align__(16) unsigned char rs_dyn[];
   KT* s_keys = reinterpret_cast<KT*>(rs_dyn);                                    // RS_TILE keys
   uint32_t* s_vals = reinterpret_cast<uint32_t*>(rs_dyn + RS_TILE * sizeof(KT));  // RS_TILE values
   const KT* keysIn = static_cast<const KT*>(a.keysIn);
   KT* keysOut = static_cast<KT*>(a.keysOut);
-  __shared__ uint32_t s_whist[RS_WARPS][256];
-  __shared__ uint32_t s_count[256];     // this block's count per digit
-  __shared__ uint32_t s_run[256];       // the same, kept for the look-back
-  __shared__ uint32_t s_local[256];     // exclusive prefix of s_count over digits
-  __shared__ uint32_t s_gbase[256];     // global start of this block's run per digit
-  __shared__ uint32_t s_dbase[256];     // exclusive scan of the pass histogram
-  __shared__ uint32_t s_warp[33];
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_match[ORM ? RS_WARPS : 1][256];  // OR form: per warp, lanes holding each digit
+  auto& s_whist = sh.whist;
+  auto& s_count = sh.count;
+  auto& s_run = sh.run;
+  auto& s_local = sh.local;
+  auto& s_gbase = sh.gbase;
+  auto& s_dbase = sh.dbase;
+  auto& s_warp = sh.warp;
+  auto& s_tile = sh.tile;
+  auto& s_match = sh.match;
 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const uint32_t N = *a.nItems;
@@ -479,6 +490,19 @@ __global__ void __launch_bounds__(RS_THREADS, GS_SORT_MIN_BLOCKS) k_onesweep(One
   }
 }
 
+#ifndef GS_SORT_MIN_BLOCKS
+#define GS_SORT_MIN_BLOCKS 3  // resident blocks per SM the register allocation must allow
+#endif
+// Up to RS_SMALL entries the blocks are a quarter of the size: a pass over so
+// few is one block's latency, most of it the ranking of a thread's entries one
+// after another.
+template <typename KT, bool DROP = false, bool ORM = false>
+__global__ void __launch_bounds__(RS_THREADS, GS_SORT_MIN_BLOCKS) k_onesweep(OnesweepArgs a) {
+  __shared__ OnesweepShared<ORM> sh;
+  if (*a.nItems <= RS_SMALL && a.smallBlocks) onesweep_body<KT, DROP, ORM, RS_ITEMS / 4>(a, sh);
+  else onesweep_body<KT, DROP, ORM, RS_ITEMS>(a, sh);
+}
+
 template <typename KT>
 constexpr size_t rs_dyn_smem() { return (size_t)RS_TILE * (sizeof(KT) + 4); }
 
@@ -539,6 +563,7 @@ static void radix_sort_t(const RadixSortArgs& a, cudaStream_t s) {
     o.epoch = a.epoch;
     o.pass = p;
     o.spinLimit = LOOKBACK_SPIN_LIMIT;
+    o.smallBlocks = 1;
     const bool orForm = sizeof(KT) == 4 && ((a.orPasses >> p) & 1u);
     if (o.dropAllOnes && orForm)
       k_onesweep<uint32_t, true, true><<<a.sweepGrid, RS_THREADS, rs_dyn_smem<uint32_t>(), s>>>(o);
@@ -594,6 +619,7 @@ int debug_lookback_timeout(int device, uint32_t spinLimit, uint32_t* statusOut, 
     o.nItems = small + 2058; o.hist = small; o.tileCounter = small + 2048; o.status = status;
     o.statusWord = small + 2056; o.epoch = small + 2057; o.pass = 0; o.spinLimit = spinLimit;
     o.dropAllOnes = 0;
+    o.smallBlocks = 0;
     cudaFuncSetAttribute(k_onesweep<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)rs_dyn_smem<uint32_t>());
     cudaEventRecord(e0, s);

@@ -10,6 +10,7 @@
 // once per step shape (number of views, their resolutions, splat count).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -32,7 +33,7 @@ struct StepParams {
   uint32_t gridBase[MAXB];
   DevCam cams[MAXB];
 };
-static_assert(sizeof(StepParams) % 4 == 0, "step parameters are copied as words");
+static_assert(sizeof(StepParams) % 4 == 0 && sizeof(StepParams) <= 3 * 256 * 4, "k_step_begin copies them as words");
 
 thread_local std::string g_createError;
 
@@ -440,7 +441,8 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
   GS_AL(h->vals[0], h->capacity);
   GS_AL(h->vals[1], h->capacity);
   GS_AL(h->small, (size_t)4096);
-  GS_AL(h->lbStatus, (size_t)(std::max<uint64_t>(h->capacity, (uint64_t)B * cap) / SORT_BLOCK_ENTRIES + 2) * 256);
+  const size_t lbWords = (size_t)(sort_status_blocks(std::max<uint64_t>(h->capacity, (uint64_t)B * cap)) + 2) * 256;
+  GS_AL(h->lbStatus, lbWords);
   GS_AL(h->scanPartials, (size_t)B * cap / EXPAND_BLOCK + 4);  // padded: scanned four words at a time
   GS_AL(h->outImg, (size_t)B * h->maxPix);
   GS_AL(h->finalT, (size_t)B * h->maxPix);
@@ -486,7 +488,7 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
   }
   GS_CK(cudaMemsetAsync(h->gradP, 0, (size_t)B * cap * GP_STRIDE * 4, s));
   GS_CK(cudaMemsetAsync(h->small, 0, 4096 * 4, s));
-  GS_CK(cudaMemsetAsync(h->lbStatus, 0, (size_t)(std::max<uint64_t>(h->capacity, (uint64_t)B * cap) / SORT_BLOCK_ENTRIES + 2) * 256 * 8, s));
+  GS_CK(cudaMemsetAsync(h->lbStatus, 0, lbWords * 8, s));
   // targets packed on the device, one camera at a time through a scratch
   // buffer of the largest image
   {
@@ -671,7 +673,8 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
     StepBeginArgs ba{};
     ba.ring = reinterpret_cast<const uint32_t*>(h->hRing);
     ba.slots = RING;
-    ba.words = (uint32_t)(sizeof(StepParams) / 4);
+    ba.stride = (uint32_t)(sizeof(StepParams) / 4);
+    ba.words = (uint32_t)(offsetof(StepParams, cams) + (size_t)V * sizeof(DevCam)) / 4;  // the pass's views only
     ba.seq = h->small + SMALL_SEQ;
     ba.params = reinterpret_cast<uint32_t*>(h->dParams);
     ba.nItems = nItems;
