@@ -266,7 +266,7 @@ int export_ply_records(const float* params, const float* sh, uint32_t n, uint32_
                        cudaStream_t s);
 int debug_lookback_timeout(int device, uint32_t spinLimit, uint32_t* statusOut, double* msOut);
 void launch_radix_sort(const RadixSortArgs& a, cudaStream_t s);
-void launch_raster(const RasterArgs& a, bool train, int tile, unsigned grid, int sms, cudaStream_t s);
+void launch_raster(const RasterArgs& a, bool train, int tile, unsigned grid, cudaStream_t s);
 unsigned raster_grid(uint32_t items, int sms, int perSm);
 void launch_raster_stored(const RasterArgs& a, int tile, int batchDepth, unsigned grid, cudaStream_t s);
 int raster_blocks_per_sm(int tile, bool train);

@@ -457,23 +457,27 @@ struct StagedRec {
 // Entries past the slice (cacheCap of them fit) are recomputed from the list.
 // The ten integer sums of an entry go from the warp straight to gradP.
 //
+// The backward takes two entries at a time and the forward is unrolled by
+// two, so that one entry's chain of dependent instructions runs under the
+// other's; that needs 96 registers, so 5 blocks (20 warps) per SM.  One entry at
+// a time with 72 registers and 7 blocks is 1.2% slower on full grids and 5-9%
+// slower where a few long blocks decide the time (an evaluation pass, one
+// 1080p view: 6830 -> 6506 us; 555x419, 180k splats: 7009 -> 6376 us).
+//
 // What bounds it: instruction issue (70% active), with the conversions to
 // integers (F2I: 8 cycles a warp) at 55% of their pipe and FMA at 57%.  Measured
-// on 1M splats, two 1080p views: 2.06 ms, 1.62 G warp instructions; the block
-// per tile of four warps it replaced, which met at a barrier every batch and
-// recomputed G: 2.49 ms, 2.08 G.  The cache moves 3.1 GB through DRAM in that
-// time (1.5 TB/s), loads two entries ahead; without it the pass is 9% slower.
-//
-// MINB: resident blocks per SM that the registers allow.  7 (72 registers) is
-// best while there is enough work to keep every SM full, and 5 (80 registers)
-// when fewer blocks run (raster_grid).
-template <int TILE, bool MASKED, bool BWD, int MINB>
-__global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs a) {
+// on 1M splats, two 1080p views, one entry at a time: 2.06 ms, 1.62 G warp
+// instructions; the block per tile of four warps it replaced, which met at a
+// barrier every batch and recomputed G: 2.49 ms, 2.08 G.  The cache's traffic
+// goes through DRAM (3.1 GB in that pass, 1.5 TB/s), loaded two entries ahead;
+// without the cache the pass is 9% slower.
+template <int TILE, bool MASKED, bool BWD>
+__global__ void __launch_bounds__(RW_WARPS * 32, BWD ? 5 : 6) k_raster_warp(RasterArgs a) {
   constexpr int SUB = (TILE / 8) * (TILE / 8);  // 8x8 blocks per tile
   constexpr int SPR = TILE / 8;                 // of them in one row
   static_assert(!MASKED || TILE <= 16, "entry values carry at most four block bits");
   __shared__ StagedRec s_rec[RW_WARPS][2][32];
-  __shared__ __align__(128) int32_t s_stage[BWD ? RW_WARPS : 1][2][16];
+  __shared__ __align__(256) int32_t s_stage[BWD ? RW_WARPS : 1][4][16];
   __shared__ uint32_t s_stat[3];
   __shared__ int32_t s_cam[MAX_VIEWS][2];
 
@@ -487,7 +491,7 @@ __global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs 
   if (BWD) {
     if (threadIdx.x < 3) s_stat[threadIdx.x] = 0u;
     if (threadIdx.x < 2 * MAX_VIEWS) (&s_cam[0][0])[threadIdx.x] = 0;
-    if (threadIdx.x < RW_WARPS * 2) s_stage[threadIdx.x >> 1][threadIdx.x & 1][10] = 0;  // word 10 of each row
+    if (threadIdx.x < RW_WARPS * 4) s_stage[threadIdx.x >> 2][threadIdx.x & 3][10] = 0;  // word 10 of each row
     __syncthreads();
   }
   const uint32_t warp = blockIdx.x * RW_WARPS + (uint32_t)wid;
@@ -580,6 +584,7 @@ __global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs 
         uint32_t hit = 0;
         uint32_t kA = 0, kB = 0;  // last entry of the chunk that each pixel composited
         const StagedRec* sr = s_rec[wid][b];
+#pragma unroll 2
         for (uint32_t k = 0; k < n; ++k, ++sr) {
           const float4 r0 = sr->rec.r0;
           const float4 r1 = sr->rec.r1;
@@ -727,14 +732,15 @@ __global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs 
     float2 Ta = T;
     int32_t* gradP = a.gradP + (size_t)v * a.n * GP_STRIDE + lane;
     asm volatile("mov.u64 %0, %1;" : "=l"(gradP) : "l"(gradP));  // opaque: not formed anew per entry
-    uint32_t row = smem_addr(s_stage[wid][0]);  // the staging row in use; the other is 64 bytes away
+    uint32_t row = smem_addr(s_stage[wid][0]);  // the staging rows in use: this one and the one 64 bytes on
     uint32_t slotOff;                            // this lane's word of a row
     asm volatile("mov.u32 %0, %1;" : "=r"(slotOff) : "r"((lane < 10 ? lane : 10) * 4));
     // One composited entry at shared address sr, G the pixels' exponentials (0
     // where a pixel does not composite it).  FAST: every product is finite and
     // within +-1e9, so a pixel with G = 0 or without a target (gC = 0)
-    // contributes zeros without being masked.
-    auto backward = [&](uint32_t sr, float2 G, auto FAST) {
+    // contributes zeros without being masked.  Advances Ta and S and returns
+    // the lane's ten integer values.
+    auto backward = [&](uint32_t sr, float2 G, auto FAST, int32_t q[10]) {
       const float4 r0 = lds4(sr);
       const float4 r1 = lds4(sr + 16);
       const float4 r2 = lds4(sr + 32);
@@ -780,21 +786,29 @@ __global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs 
       S1 = __ffma2_rn(bc2(r1.w), aT, S1);
       S2 = __ffma2_rn(bc2(r2.x), aT, S2);
       Ta = Tb;
-      // the 10 sums (every lane has them) go through shared memory, and lanes
-      // 0-9 add one each to the splat's slots; two staging rows in turn, so
-      // one barrier an entry is enough
-      int32_t q[10];
 #pragma unroll
       for (int k = 0; k < 10; ++k) q[k] = __float2int_rz(xs[k].x) + __float2int_rz(xs[k].y);
-      sts4(row, __reduce_add_sync(FULL, q[0]), __reduce_add_sync(FULL, q[1]), __reduce_add_sync(FULL, q[2]),
+    };
+    // The ten sums over the warp (every lane has them) go through shared memory,
+    // and lanes 0-9 add one each to the splat's slots.
+    auto put = [&](uint32_t at, const int32_t q[10]) {
+      sts4(at, __reduce_add_sync(FULL, q[0]), __reduce_add_sync(FULL, q[1]), __reduce_add_sync(FULL, q[2]),
            __reduce_add_sync(FULL, q[3]));
-      sts4(row + 16, __reduce_add_sync(FULL, q[4]), __reduce_add_sync(FULL, q[5]), __reduce_add_sync(FULL, q[6]),
+      sts4(at + 16, __reduce_add_sync(FULL, q[4]), __reduce_add_sync(FULL, q[5]), __reduce_add_sync(FULL, q[6]),
            __reduce_add_sync(FULL, q[7]));
-      sts2(row + 32, __reduce_add_sync(FULL, q[8]), __reduce_add_sync(FULL, q[9]));
+      sts2(at + 32, __reduce_add_sync(FULL, q[8]), __reduce_add_sync(FULL, q[9]));
+    };
+    auto add = [&](uint32_t at, uint32_t sr) {  // lanes from 10 on read word 10, which stays 0
+      red_nz(gradP + (size_t)lds1(sr + 48) * GP_STRIDE, (int32_t)lds1(at + slotOff));
+    };
+    // one barrier per entry (or pair): the rows alternate with those 128 bytes away
+    auto one = [&](uint32_t sr, float2 G, auto FAST) {
+      int32_t q[10];
+      backward(sr, G, FAST, q);
+      put(row, q);
       __syncwarp();
-      // lanes from 10 on read word 10, which stays 0
-      red_nz(gradP + (size_t)lds1(sr + 48) * GP_STRIDE, (int32_t)lds1(row + slotOff));
-      row ^= 64u;
+      add(row, sr);
+      row ^= 128u;
     };
     // list entries past the cache: recompute the exponentials chunk by chunk
     if (uncached < e) {
@@ -817,7 +831,7 @@ __global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs 
           const bool c2a = j < endA && ee.x <= E_CUT && araw.x >= A_MIN;
           const bool c2b = j < endB && ee.y <= E_CUT && araw.y >= A_MIN;
           if (__any_sync(FULL, c2a || c2b))
-            backward(smem_addr(sr), make_float2(c2a ? G.x : 0.0f, c2b ? G.y : 0.0f), std::false_type{});
+            one(smem_addr(sr), make_float2(c2a ? G.x : 0.0f, c2b ? G.y : 0.0f), std::false_type{});
         }
         __syncwarp();
       }
@@ -851,13 +865,30 @@ __global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs 
         const StagedRec* sr = s_rec[wid][b];
         widen(sr, n);
         auto chunk = [&](auto FAST) {
+          constexpr uint32_t STEP = (uint32_t)sizeof(StagedRec);
           uint32_t at = smem_addr(sr);
-          for (const uint32_t end = at + n * (uint32_t)sizeof(StagedRec); at != end; at += (uint32_t)sizeof(StagedRec)) {
+          const uint32_t end = at + n * STEP;
+          for (; end - at >= 2u * STEP; at += 2u * STEP) {
+            int32_t q0[10], q1[10];
+            const float2 A = G0, B = G1;
+            G0 = __ldcg(gl - 64);
+            G1 = __ldcg(gl - 96);
+            gl -= 64;
+            backward(at, A, FAST, q0);
+            backward(at + STEP, B, FAST, q1);
+            put(row, q0);
+            put(row + 64u, q1);
+            __syncwarp();
+            add(row, at);
+            add(row + 64u, at + STEP);
+            row ^= 128u;
+          }
+          for (; at != end; at += STEP) {
             const float2 G = G0;
             G0 = G1;
             G1 = __ldcg(gl - 64);
             gl -= 32;
-            backward(at, G, FAST);
+            one(at, G, FAST);
           }
         };
         if (fast) chunk(std::true_type{});
@@ -878,15 +909,14 @@ __global__ void __launch_bounds__(RW_WARPS * 32, MINB) k_raster_warp(RasterArgs 
   }
 }
 
-// wide: the build with more registers a thread, for grids of at most 5 blocks per SM
-static const void* warp_kernel(int tile, bool masked, bool train, bool wide) {
-  if (tile == 8) return train ? (const void*)k_raster_warp<8, false, true, 6> : (const void*)k_raster_warp<8, false, false, 8>;
-  if (tile == 32)
-    return train ? (const void*)k_raster_warp<32, false, true, 6> : (const void*)k_raster_warp<32, false, false, 8>;
-  if (!masked)
-    return train ? (const void*)k_raster_warp<16, false, true, 6> : (const void*)k_raster_warp<16, false, false, 8>;
-  if (!train) return (const void*)k_raster_warp<16, true, false, 8>;
-  return wide ? (const void*)k_raster_warp<16, true, true, 5> : (const void*)k_raster_warp<16, true, true, 7>;
+template <int TILE, bool MASKED>
+static const void* warp_kernel(bool train) {
+  return train ? (const void*)k_raster_warp<TILE, MASKED, true> : (const void*)k_raster_warp<TILE, MASKED, false>;
+}
+static const void* warp_kernel(int tile, bool masked, bool train) {
+  if (tile == 8) return warp_kernel<8, false>(train);
+  if (tile == 32) return warp_kernel<32, false>(train);
+  return masked ? warp_kernel<16, true>(train) : warp_kernel<16, false>(train);
 }
 
 template <int TILE>
@@ -905,38 +935,33 @@ void launch_raster_stored(const RasterArgs& a, int tile, int batchDepth, unsigne
   else launch_stored<16>(a, batchDepth, grid, s);
 }
 
-void launch_raster(const RasterArgs& a, bool train, int tile, unsigned grid, int sms, cudaStream_t s) {
+void launch_raster(const RasterArgs& a, bool train, int tile, unsigned grid, cudaStream_t s) {
   if (grid == 0) return;
   RasterArgs copy = a;
   void* args[] = {&copy};
-  cudaLaunchKernel(warp_kernel(tile, a.idMask != 0xFFFFFFFFu, train, grid <= 5u * (unsigned)sms), dim3(grid),
-                   dim3(RW_WARPS * 32), args, 0, s);
+  cudaLaunchKernel(warp_kernel(tile, a.idMask != 0xFFFFFFFFu, train), dim3(grid), dim3(RW_WARPS * 32), args, 0, s);
 }
 
 int raster_blocks_per_sm(int tile, bool train) {
-  int least = 64;
-  for (int k = 0; k < 4; ++k) {
-    if (k == 3 && train) continue;  // the wide build runs on smaller grids only
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, warp_kernel(tile, (k & 1) != 0, train, (k & 2) != 0),
-                                                  RW_WARPS * 32, 0);
-    if (n < least) least = n;
-  }
-  return least < 1 ? 1 : least;
+  int a = 0, b = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, warp_kernel(tile, false, train), RW_WARPS * 32, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, warp_kernel(tile, true, train), RW_WARPS * 32, 0);
+  const int perSm = std::min(a, b);
+  return perSm < 1 ? 1 : perSm;
 }
 
 // Blocks of the persistent raster over `items` 8x8 blocks.  The longest tiles
-// are taken first, and with every warp slot filled they share an SM with 27
+// are taken first, and with every warp slot filled they share an SM with 19
 // others and finish last, so when there are only a few items per slot fewer
-// blocks are launched: about 5.3 items a warp, at least 3 blocks per SM.
-// Train passes at 7 / 6 / 5 / 4 / 3 blocks per SM, us a pass: 3780 items
-// 8995 / 8938 / 8696 / 8218 / 7797; 10032 items 14020 / 13801 / 13211 / 12582 /
-// 12827; 15504 items 8870 / 8734 / 8452 / 8601 / 9325; 32640 items 47788 /
-// 48405 / 50258 / 53515 / 58853.
+// blocks are launched: about 5.3 items a warp, at least 2 blocks per SM.
+// Train passes at 5 / 4 / 3 / 2 blocks per SM, us a pass of the same steps:
+// 3780 items 6987 / 6679 / 6322 / 5970; 10032 items 11862 / 11635 / 11796 /
+// 12813; 15504 items 7239 / 7332 / 8071 / 9583; 32640 items 45740 / 48037 /
+// 52569 / 63085.
 unsigned raster_grid(uint32_t items, int sms, int perSm) {
   const unsigned all = (items + RW_WARPS - 1) / RW_WARPS;
   const double k = std::ceil((double)items / (5.3 * RW_WARPS * sms));
-  const unsigned blocks = (unsigned)(std::min((double)perSm, std::max(3.0, k)) * sms);
+  const unsigned blocks = (unsigned)(std::min((double)perSm, std::max(2.0, k)) * sms);
   return all < blocks ? all : blocks;
 }
 

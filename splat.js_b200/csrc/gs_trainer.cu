@@ -853,7 +853,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
     unsigned grid = ceil_div(rasterItems, RW_WARPS);
     if (persistent) grid = raster_grid(rasterItems, h->sms, perSm);
     if (persistent && train) grid = std::min(grid, h->cacheWarps / RW_WARPS);  // a slice for every warp
-    launch_raster(rr, train, sh.tile, grid, h->sms, s);
+    launch_raster(rr, train, sh.tile, grid, s);
   }
   if (h->profiling) cudaEventRecord(ph[3], s);
 
