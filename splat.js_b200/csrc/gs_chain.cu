@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256) k_visible_list(ChainArgs a, uint32_t bloc
 // the view's camera; the result -- the 14 parameter gradients, the gated
 // colour gradient dRGB and the view direction (from which the SH basis Y is
 // recomputed) -- goes to viewGrad[slot] for pass 2.  Camera gradients are
-// summed per warp in fixed point (order-independent) with one atomic each.
+// summed per block in fixed point (order-independent) with one atomic each.
 template <int DEG>
 __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainArgs a) {
   using Rows = ShRows<DEG>;
@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainAr
   // global memory around every store); every thread issues its own loads
   // before the barrier that publishes it
   __shared__ DevCam s_cam;
+  __shared__ uint32_t s_cg[4][7];
   copy_cams(&s_cam, a.cams + v, 1);
   // each warp copies the SH rows of its own items, whole rows by neighbouring lanes
   __shared__ __align__(16) float s_sh[K > 0 ? 128 * Rows::PITCH : 4];
@@ -383,16 +384,18 @@ __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainAr
       o[4] = make_float4(dRGB[2], vd[0], vd[1], vd[2]);
     }
   }
-  // camera gradients: warp sums of the fixed-point values, one atomic each
+  // camera gradients: block sums of the fixed-point values, one atomic each
   if (c.train) {
     const float cv[7] = {cg.w[0], cg.w[1], cg.w[2], cg.t[0], cg.t[1], cg.t[2], cg.logf};
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
       const uint32_t r = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)fixq(cv[k], FIXCAM));
-      if (lane == 0 && r) {
-        const uint32_t idx = k < 6 ? c.camIdx * 8u + (uint32_t)k : c.ncams * 8u;
-        atomicAdd(&a.gradCam[idx], (int32_t)r);
-      }
+      if (lane == 0) s_cg[threadIdx.x >> 5][k] = r;
+    }
+    __syncthreads();
+    if (threadIdx.x < 7) {
+      const uint32_t k = threadIdx.x, r = s_cg[0][k] + s_cg[1][k] + s_cg[2][k] + s_cg[3][k];
+      if (r) atomicAdd(&a.gradCam[k < 6 ? c.camIdx * 8u + k : c.ncams * 8u], (int32_t)r);
     }
   }
 }

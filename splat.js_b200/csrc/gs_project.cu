@@ -167,11 +167,11 @@ __global__ void __launch_bounds__(PROJECT_THREADS, 8) k_project(ProjectArgs a) {
 
     // tile bounds (shaders.js:303-308)
     const int tx = c.tilesX, ty = c.tilesY;
-    const float TF = (float)a.tile;
-    const uint32_t x0 = u32sat(clampf(floorf((mx - rad) / TF), 0.0f, (float)(tx - 1)));
-    const uint32_t x1 = u32sat(clampf(floorf((mx + rad) / TF), 0.0f, (float)(tx - 1)));
-    const uint32_t y0 = u32sat(clampf(floorf((my - rad) / TF), 0.0f, (float)(ty - 1)));
-    const uint32_t y1 = u32sat(clampf(floorf((my + rad) / TF), 0.0f, (float)(ty - 1)));
+    const float rTF = 1.0f / (float)a.tile;  // the tile is a power of two: multiplying is the same as dividing
+    const uint32_t x0 = u32sat(clampf(floorf((mx - rad) * rTF), 0.0f, (float)(tx - 1)));
+    const uint32_t x1 = u32sat(clampf(floorf((mx + rad) * rTF), 0.0f, (float)(tx - 1)));
+    const uint32_t y0 = u32sat(clampf(floorf((my - rad) * rTF), 0.0f, (float)(ty - 1)));
+    const uint32_t y1 = u32sat(clampf(floorf((my + rad) * rTF), 0.0f, (float)(ty - 1)));
     a.rect[slot] = make_uint2(x0 | (y0 << 16), x1 | (y1 << 16));
     // cull parameters: the tile cull and the rasteriser's warp-block masks
     const float4 cq = cullParams(mx, my, r.r0.z, r.r0.w, r.r1.x, r.r1.y, a.aMin, a.eCut, x0, x1, y0, y1, a.tile);
@@ -385,6 +385,12 @@ __device__ __forceinline__ uint32_t band_columns(const float4 cq, float mx, floa
   if (r < 0) return 1u;
   return (uint32_t)l | ((uint32_t)r << 16);
 }
+// columns 0-31 of a band as bits
+__device__ __forceinline__ uint32_t column_mask(uint32_t b) {
+  const uint32_t first = b & 0xFFFFu, last = b >> 16;
+  if (first > 31u || first > last) return 0u;
+  return (last >= 31u ? 0xFFFFFFFFu : (2u << last) - 1u) & (0xFFFFFFFFu << first);
+}
 // block bits of a tile whose left block column is col: bands b0 (rows 0-7), b1
 __device__ __forceinline__ uint32_t block_bits(uint32_t b0, uint32_t b1, uint32_t col) {
   uint32_t m = 0;
@@ -576,8 +582,17 @@ __global__ void __launch_bounds__(256) k_expand(ExpandArgs a) {
       if (dense && chunk <= EXPAND_STAGE) {
         uint2* st = s_out[threadIdx.x >> 5];
         uint32_t at = inc - cnt;  // rows follow one another in output order
-        for (uint32_t j = 0; j < cnt; ++j, ++at)
-          st[at] = make_uint2(rowKey + j, oi | (a.masks ? block_bits(band0, band1, 2u * j) : 0u));
+        if (cnt <= 16u) {  // the row's block columns as two 32-bit masks, two bits an entry
+          uint32_t m0 = a.masks ? column_mask(band0) : 0u, m1 = a.masks ? column_mask(band1) : 0u;
+          for (uint32_t j = 0; j < cnt; ++j, ++at) {
+            st[at] = make_uint2(rowKey + j, oi | (((m0 & 3u) | (m1 & 3u) << 2) << ID_BITS));
+            m0 >>= 2;
+            m1 >>= 2;
+          }
+        } else {
+          for (uint32_t j = 0; j < cnt; ++j, ++at)
+            st[at] = make_uint2(rowKey + j, oi | (a.masks ? block_bits(band0, band1, 2u * j) : 0u));
+        }
         __syncwarp();
         for (uint32_t k = (uint32_t)lane; k < chunk; k += 32) {
           const uint2 kv = st[k];
