@@ -272,23 +272,36 @@ __device__ __forceinline__ float adam_g(float g) { return fabsf(g) < 1e18f ? g :
 // order inside a list follows the blocks' atomics (roughly ascending), which
 // pass 1 uses only for memory locality: each item's results go to its own
 // slot and camera gradients are integer sums, so no result depends on it.
+// A block takes PER strips of 256 splats: the atomics of all blocks go to the
+// views' counters, one cache sector, one after another, and with one strip
+// they were the whole time (42 us for 8 views of 1M splats); below 256k splats
+// one strip spreads the work over more SMs.
+template <int PER>
 __global__ void __launch_bounds__(256) k_visible_list(ChainArgs a, uint32_t blocksPerView) {
-  __shared__ uint32_t s_warp[8];
+  __shared__ uint32_t s_warp[8 * PER];
   __shared__ uint32_t s_base;
   const uint32_t v = blockIdx.x / blocksPerView;
-  const uint32_t i = (blockIdx.x - v * blocksPerView) * blockDim.x + threadIdx.x;
+  const uint32_t i0 = (blockIdx.x - v * blocksPerView) * (256u * PER) + threadIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const bool vis = i < a.n && a.rect[(size_t)v * a.n + i].x != 0xFFFFFFFFu;
-  const uint32_t b = __ballot_sync(0xFFFFFFFFu, vis);
-  if (lane == 0) s_warp[wid] = (uint32_t)__popc(b);
+  uint32_t b[PER];
+#pragma unroll
+  for (int r = 0; r < PER; ++r) {
+    const uint32_t i = i0 + 256u * r;
+    b[r] = __ballot_sync(0xFFFFFFFFu, i < a.n && a.rect[(size_t)v * a.n + i].x != 0xFFFFFFFFu);
+    if (lane == 0) s_warp[r * 8 + wid] = (uint32_t)__popc(b[r]);
+  }
   __syncthreads();
   if (threadIdx.x == 0) {  // one atomic per block
     uint32_t t = 0;
-    for (int w = 0; w < 8; ++w) { const uint32_t c = s_warp[w]; s_warp[w] = t; t += c; }
+    for (int w = 0; w < 8 * PER; ++w) { const uint32_t c = s_warp[w]; s_warp[w] = t; t += c; }
     s_base = t ? atomicAdd(&a.visCount[v], t) : 0u;
   }
   __syncthreads();
-  if (vis) a.visList[(size_t)v * a.n + s_base + s_warp[wid] + (uint32_t)__popc(b & ((1u << lane) - 1u))] = i;
+#pragma unroll
+  for (int r = 0; r < PER; ++r)
+    if ((b[r] >> lane) & 1u)
+      a.visList[(size_t)v * a.n + s_base + s_warp[r * 8 + wid] + (uint32_t)__popc(b[r] & ((1u << lane) - 1u))] =
+          i0 + 256u * r;
 }
 
 // Pass 1: one thread per visible (view, splat) item of the lists above.
@@ -299,30 +312,37 @@ __global__ void __launch_bounds__(256) k_visible_list(ChainArgs a, uint32_t bloc
 // the view's camera; the result -- the 14 parameter gradients, the gated
 // colour gradient dRGB and the view direction (from which the SH basis Y is
 // recomputed) -- goes to viewGrad[slot] for pass 2.  Camera gradients are
-// summed per block in fixed point (order-independent) with one atomic each.
+// summed per block in fixed point (order-independent) with one atomic each.  A
+// block takes chainStrips strips of 128 items, to send fewer of those.  Per-warp
+// atomics were what bounded the pass: 765 us for 8 views of 1M splats, 527 us
+// with one per block of 128.
 template <int DEG>
 __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainArgs a) {
   using Rows = ShRows<DEG>;
   constexpr int K = Rows::K;
-  const uint32_t sb = blockIdx.x / (uint32_t)a.V;
-  const int v = (int)(blockIdx.x - sb * (uint32_t)a.V);
-  const uint32_t pos = sb * blockDim.x + threadIdx.x;
+  const uint32_t sb0 = blockIdx.x / (uint32_t)a.V;
+  const int v = (int)(blockIdx.x - sb0 * (uint32_t)a.V);
   const uint32_t cnt = a.visCount[v];
-  if (sb * blockDim.x >= cnt) return;  // the whole block is past the list (uniform)
-  const bool have = pos < cnt;
-  const uint32_t i = have ? a.visList[(size_t)v * a.n + pos] : 0u;
+  uint32_t pos = sb0 * a.chainStrips * blockDim.x + threadIdx.x;
+  if (pos - threadIdx.x >= cnt) return;  // the whole block is past the list (uniform)
   const int lane = threadIdx.x & 31;
   // the block's camera in shared memory (read once, not re-fetched from
-  // global memory around every store); every thread issues its own loads
-  // before the barrier that publishes it
+  // global memory around every store)
   __shared__ DevCam s_cam;
   __shared__ uint32_t s_cg[4][7];
-  copy_cams(&s_cam, a.cams + v, 1);
-  // each warp copies the SH rows of its own items, whole rows by neighbouring lanes
   __shared__ __align__(16) float s_sh[K > 0 ? 128 * Rows::PITCH : 4];
+  copy_cams(&s_cam, a.cams + v, 1);
+  __syncthreads();
+  const DevCam& c = s_cam;
   float* const warpRows = s_sh + (K > 0 ? (threadIdx.x & ~31u) * Rows::PITCH : 0);
+  uint32_t cgSum[7] = {0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  for (uint32_t strip = 0; strip < a.chainStrips && pos - lane < cnt; ++strip, pos += blockDim.x) {
+  const bool have = pos < cnt;
+  const uint32_t i = have ? a.visList[(size_t)v * a.n + pos] : 0u;
+  // each warp copies the SH rows of its own items, whole rows by neighbouring lanes
   if (K > 0) {
     constexpr int PART = DEG == 2 ? 4 : 1, PARTS = K > 0 ? Rows::WORDS / PART : 1;  // words per copy, copies per row
+    __syncwarp();  // the rows of the strip before have been read
 #pragma unroll 5
     for (int j = 0; j < PARTS; ++j) {
       const int e = lane + 32 * j, row = e / PARTS, col = (e - row * PARTS) * PART;
@@ -347,8 +367,7 @@ __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainAr
     }
   }
   cp_async_wait<0>();
-  __syncthreads();
-  const DevCam& c = s_cam;
+  __syncwarp();
   CamGrad7 cg = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, 0.0f};
   if (have) {
     {
@@ -384,14 +403,18 @@ __global__ void __launch_bounds__(128, GS_CHAIN_MIN_BLOCKS) k_chain_view(ChainAr
       o[4] = make_float4(dRGB[2], vd[0], vd[1], vd[2]);
     }
   }
-  // camera gradients: block sums of the fixed-point values, one atomic each
+  // camera gradients: fixed-point sums (order-independent)
   if (c.train) {
     const float cv[7] = {cg.w[0], cg.w[1], cg.w[2], cg.t[0], cg.t[1], cg.t[2], cg.logf};
 #pragma unroll
-    for (int k = 0; k < 7; ++k) {
-      const uint32_t r = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)fixq(cv[k], FIXCAM));
-      if (lane == 0) s_cg[threadIdx.x >> 5][k] = r;
-    }
+    for (int k = 0; k < 7; ++k) cgSum[k] += __reduce_add_sync(0xFFFFFFFFu, (uint32_t)fixq(cv[k], FIXCAM));
+  }
+  }
+  // one atomic each per block: they all go to the same few cache sectors
+  if (c.train) {
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < 7; ++k) s_cg[threadIdx.x >> 5][k] = cgSum[k];
     __syncthreads();
     if (threadIdx.x < 7) {
       const uint32_t k = threadIdx.x, r = s_cg[0][k] + s_cg[1][k] + s_cg[2][k] + s_cg[3][k];
@@ -530,12 +553,20 @@ __global__ void __launch_bounds__(128) k_chain_adam(ChainArgs a) {
   }
 }
 
-void launch_chain_adam(const ChainArgs& a, int deg, cudaStream_t s) {
+void launch_chain_adam(const ChainArgs& args, int deg, cudaStream_t s) {
+  ChainArgs a = args;
   const unsigned blocks = (a.n + 127) / 128;
   if (blocks == 0) return;
-  const unsigned g1 = blocks * (unsigned)a.V;
-  const unsigned bpv = (a.n + 255) / 256;
-  k_visible_list<<<bpv * (unsigned)a.V, 256, 0, s>>>(a, bpv);
+  // strips per chain block: four while that leaves 16 blocks per SM
+  a.chainStrips = (uint64_t)blocks * a.V >= 4ull * 16 * 148 ? 4 : 1;
+  const unsigned g1 = (blocks + a.chainStrips - 1) / a.chainStrips * (unsigned)a.V;
+  if (a.n >= (1u << 18)) {
+    const unsigned bpv = (a.n + 2047) / 2048;
+    k_visible_list<8><<<bpv * (unsigned)a.V, 256, 0, s>>>(a, bpv);
+  } else {
+    const unsigned bpv = (a.n + 255) / 256;
+    k_visible_list<1><<<bpv * (unsigned)a.V, 256, 0, s>>>(a, bpv);
+  }
   switch (deg) {
     case 0: k_chain_view<0><<<g1, 128, 0, s>>>(a); k_chain_adam<0><<<blocks, 128, 0, s>>>(a); break;
     case 1: k_chain_view<1><<<g1, 128, 0, s>>>(a); k_chain_adam<1><<<blocks, 128, 0, s>>>(a); break;

@@ -209,6 +209,7 @@ struct ChainArgs {
   float* viewGrad;         // V * n * VIEWGRAD_STRIDE: per-(view, splat) chain results
   uint32_t* visList;       // V * n: per view, indices of the visible splats
   uint32_t* visCount;      // V counters, cleared before the step
+  uint32_t chainStrips;    // strips of 128 list items per chain block (set by the launcher)
   float anisoReg;
   int32_t* gradCam;
   float* gradF;            // optional readout (n * 16)
