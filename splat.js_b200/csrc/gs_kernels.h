@@ -43,7 +43,7 @@ struct ProjectArgs {
   int32_t* diffGrid;       // GRID_COPIES copies of: per view (tilesX+1)*(tilesY+1), cleared before
   const uint32_t* gridBase;  // V offsets into a copy
   uint32_t gridCells;      // cells of one copy (all views)
-  float4* cullRecs;        // V * n warp-block cull parameters (p, q, kA, 0)
+  float4* cullRecs;        // V * n cull parameters (p, q, kA, 0) for the raster, or null: it has block bits
   uint4* itemSrc;          // V * n * 2: per visible slot (rect, mean, cull parameters, slot) for the expansion
 };
 

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(PROJECT_THREADS, 8) k_project(ProjectArgs a) {
     a.rect[slot] = make_uint2(x0 | (y0 << 16), x1 | (y1 << 16));
     // cull parameters: the tile cull and the rasteriser's warp-block masks
     const float4 cq = cullParams(mx, my, r.r0.z, r.r0.w, r.r1.x, r.r1.y, a.aMin, a.eCut, x0, x1, y0, y1, a.tile);
-    a.cullRecs[slot] = cq;
+    if (a.cullRecs) a.cullRecs[slot] = cq;
     // what the expansion needs of this item, in one 32-byte record it
     // gathers with a single sector read
     a.itemSrc[2 * slot] = make_uint4(x0 | (y0 << 16), x1 | (y1 << 16), __float_as_uint(mx), __float_as_uint(my));

@@ -545,7 +545,7 @@ int gs_get_state(const gs_trainer* h, gs_state* out) {
   uint32_t le = 0;
   if (h->ready) cudaMemcpy(&le, h->small + 2057, 4, cudaMemcpyDeviceToHost);
   out->lastEntries = le;
-  out->stepUploadBytes = (uint32_t)sizeof(StepParams);
+  out->stepUploadBytes = (uint32_t)(offsetof(StepParams, cams) + (size_t)std::max(1, h->lastV) * sizeof(DevCam));
   out->lastLaunches = h->lastLaunches;
   return GS_OK;
 }
@@ -705,7 +705,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   pa.diffGrid = h->diffGrid;
   pa.gridCells = gridCells;
   pa.gridBase = h->dParams->gridBase;
-  pa.cullRecs = h->cullRecs;
+  pa.cullRecs = masks && !(sh.mode == 3 && sh.variant == 1) ? nullptr : h->cullRecs;
   pa.itemSrc = h->itemSrc;
   launch_project(pa, h->o.shDeg, s);
 
