@@ -93,7 +93,7 @@ struct gs_trainer {
   uint2* ranges = nullptr;
   uint32_t* viewDrops = nullptr;
   uint32_t* workOrder = nullptr;
-  uint32_t* keys[2] = {nullptr, nullptr};     // entries: global tile id
+  uint32_t* keys[2] = {nullptr, nullptr};     // entries: global tile id (one allocation; the raster's cache may use it)
   uint32_t* vals[2] = {nullptr, nullptr};     // entries: splat id
   uint64_t* pkeys[2] = {nullptr, nullptr};    // presort keys (u32 depth bits); refine's u64 donor keys
   uint32_t* pvals[2] = {nullptr, nullptr};    // presort items: slot = view * n + splat
@@ -436,8 +436,9 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
   GS_AL(h->ranges, (size_t)B * h->maxTiles);
   GS_AL(h->viewDrops, (size_t)MAXB);
   GS_AL(h->workOrder, (size_t)B * h->maxTiles);
-  GS_AL(h->keys[0], h->capacity);
-  GS_AL(h->keys[1], h->capacity);
+  const size_t keyStride = ((size_t)h->capacity + 63) & ~(size_t)63;
+  GS_AL(h->keys[0], 2 * keyStride);
+  h->keys[1] = h->keys[0] + keyStride;
   GS_AL(h->vals[0], h->capacity);
   GS_AL(h->vals[1], h->capacity);
   GS_AL(h->small, (size_t)4096);
@@ -462,7 +463,12 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
     h->cacheWarps = (uint32_t)std::min<uint64_t>((uint64_t)h->sms * perSm * RW_WARPS,
                                                  std::max<uint64_t>((uint64_t)B * blocks * 16, RW_WARPS));
     h->cacheCap = RASTER_CACHE_ENTRIES;
-    if (dalloc(h, &h->cacheG, ((size_t)h->cacheWarps * (h->cacheCap + 2) + 1) * 32) != GS_OK) {
+    const size_t slots = (size_t)h->cacheWarps * (h->cacheCap + 2) + 1;
+    if (slots * 256 <= 2 * keyStride * 4) {
+      // the entries' keys are free once the tile ranges are known: the cache
+      // lives there when it fits (small views, large entry budgets)
+      h->cacheG = reinterpret_cast<float2*>(h->keys[0]);
+    } else if (dalloc(h, &h->cacheG, slots * 32) != GS_OK) {
       cudaGetLastError();  // not an error: one slot a warp is enough to run
       h->cacheCap = 0;
       if ((rc = dalloc(h, &h->cacheG, ((size_t)h->cacheWarps * 2 + 1) * 32)) != GS_OK) { free_all(h); return rc; }
