@@ -11,13 +11,15 @@
 //      count), and a presort item: key = depth bits -- all ones when culled
 //      -- and value slot = view * n + splat;
 //   2. k_tile_counts (one block per view): tileCnt, the reference's entry
-//      budget (drops), and view-local tile ranges; k_tile_ranges_finish
-//      offsets them by the earlier views' totals;
+//      budget (drops) and, for full lists, view-local tile ranges, which
+//      k_tile_ranges_finish offsets by the earlier views' totals (culled
+//      lists take theirs from the sorted keys, k_ranges_from_keys);
 //   3. the items are radix-sorted by depth bits (stable from slot order, so
 //      equal depths keep id order; views stay interleaved);
-//   4. k_expand (count pass) / scan / k_expand (key pass) expand the sorted
-//      items into one entry per (splat, live tile) -- key = global tile id
-//      (32 bits), value = splat id -- written in that order;
+//   4. k_expand (count pass) / scan of its block totals / k_expand (key pass)
+//      expand the sorted items into one entry per (splat, live tile) -- key =
+//      global tile id (32 bits), value = splat id and, at 16-pixel tiles, the
+//      8x8 blocks it may reach -- written in that order;
 //   5. a stable radix sort on the global tile id (each id belongs to one
 //      view) leaves every tile's entries in (depth bits, id) order: the
 //      reference's per-tile order, with two passes over 8-byte entries
