@@ -318,8 +318,8 @@ __global__ void __launch_bounds__(1024) k_tile_counts(TileRangeArgs a) {
   }
 }
 
-// Offsets every view's tile ranges by the entries of the views before it and
-// writes the batch's entry total.
+// Offsets every view's tile ranges by the entries of the views before it,
+// writes the batch's entry total and counts the tiles per work-order bucket.
 __global__ void k_tile_ranges_finish(TileRangeArgs a, uint32_t totalTiles) {
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x;
   if (gt == 0) {
@@ -327,15 +327,18 @@ __global__ void k_tile_ranges_finish(TileRangeArgs a, uint32_t totalTiles) {
     for (int v = 0; v < a.V; ++v) tot += a.viewTotal[v];
     a.totalEntries[0] = tot;
   }
-  if (gt >= totalTiles) return;
-  int v = 0;
-  while (v + 1 < a.V && a.cams[v + 1].tileBase <= gt) ++v;
-  uint32_t base = 0;
-  for (int u = 0; u < v; ++u) base += a.viewTotal[u];
-  const uint2 r = a.ranges[gt];
-  a.ranges[gt] = make_uint2(r.x + base, r.y + base);
-  const uint32_t b = tile_bucket(r), peers = __match_any_sync(__activemask(), b);
-  if ((threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&a.buckets[b], (uint32_t)__popc(peers));
+  uint32_t b = 64u;  // every lane stays for the match below: lanes past the last tile hold no bucket
+  if (gt < totalTiles) {
+    int v = 0;
+    while (v + 1 < a.V && a.cams[v + 1].tileBase <= gt) ++v;
+    uint32_t base = 0;
+    for (int u = 0; u < v; ++u) base += a.viewTotal[u];
+    const uint2 r = a.ranges[gt];
+    a.ranges[gt] = make_uint2(r.x + base, r.y + base);
+    b = tile_bucket(r);
+  }
+  const uint32_t peers = __match_any_sync(0xFFFFFFFFu, b);
+  if (b < 64u && (threadIdx.x & 31u) == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&a.buckets[b], (uint32_t)__popc(peers));
 }
 
 // The live columns of one tile row of an item's rectangle.  tileLive(tx, ty)
