@@ -54,6 +54,14 @@ struct Shape {
 
 }  // namespace
 
+// What a pass's shape settles about its buffers and launches.
+struct PassLayout {
+  uint32_t totalTiles = 0, gridCells = 0;
+  int passes = 0;        // of the tile sort: the sorted entries are in buffer passes & 1
+  bool masks = false;    // entry values carry block bits
+  uint32_t launches = 0;  // kernels
+};
+
 struct gs_trainer {
   gs_options o{};
   std::string err;
@@ -130,10 +138,7 @@ struct gs_trainer {
   // ---- last raster (for introspection) ----
   int lastV = 0;
   DevCam lastCams[MAXB];
-  int lastPasses = 0;
-  bool lastMasks = false;  // entry values carry block bits
-  uint32_t lastLaunches = 0;
-  uint32_t lastTotalTiles = 0;
+  PassLayout last;
 
   // ---- refine scratch (allocated at the first refine) ----
   struct {
@@ -552,7 +557,7 @@ int gs_get_state(const gs_trainer* h, gs_state* out) {
   if (h->ready) cudaMemcpy(&le, h->small + 2057, 4, cudaMemcpyDeviceToHost);
   out->lastEntries = le;
   out->stepUploadBytes = (uint32_t)(offsetof(StepParams, cams) + (size_t)std::max(1, h->lastV) * sizeof(DevCam));
-  out->lastLaunches = h->lastLaunches;
+  out->lastLaunches = h->last.launches;
   return GS_OK;
 }
 
@@ -590,6 +595,29 @@ static int bits_for(uint32_t x) {  // bits needed to hold values 0..x
   int b = 1;
   while (b < 32 && (x >> b) != 0) ++b;
   return b;
+}
+
+// Entry values carry 8x8 block bits above the splat id (k_expand) when the
+// tile is 16 pixels (four blocks) and the ids leave four bits free.
+static bool block_masks(int tile, uint32_t n) { return tile == 16 && n <= (1u << ID_BITS); }
+
+constexpr int PRESORT_PASSES = 4;  // byte digits of the depth bits
+
+static PassLayout pass_layout(const gs_trainer* h, const Shape& sh) {
+  PassLayout p;
+  for (int v = 0; v < sh.V; ++v) {
+    const uint32_t tx = ceil_div((uint32_t)sh.w[v], (uint32_t)sh.tile), ty = ceil_div((uint32_t)sh.h[v], (uint32_t)sh.tile);
+    p.totalTiles += tx * ty;
+    p.gridCells += (tx + 1) * (ty + 1);
+  }
+  p.passes = (bits_for(p.totalTiles ? p.totalTiles - 1 : 0) + 7) / 8;
+  p.masks = block_masks(sh.tile, sh.n);
+  // begin, project, tile counts [+ finish], presort (histogram + passes),
+  // entry counts, scan, entry keys, tile sort (histogram + passes),
+  // [ranges from keys], [work order], raster, [visible lists, chain per view, sum + Adam]
+  p.launches = (sh.cull ? 3u : 4u) + 1u + (uint32_t)PRESORT_PASSES + 1u + 1u + 1u + 1u + (uint32_t)p.passes +
+               (sh.cull ? 1u : 0u) + (h->o.persistent ? 1u : 0u) + 1u + (sh.chain ? 3u : 0u);
+  return p;
 }
 
 // Fills the next ring slot with the views' records and the Adam parameters.
@@ -630,15 +658,12 @@ static int begin_pass(gs_trainer* h) {
   }
   return GS_OK;
 }
-static void end_pass(gs_trainer* h) {
+static void end_pass(gs_trainer* h, const Shape& sh) {
   cudaEventRecord(h->ringEv[h->seq % RING], h->stream);
   ++h->seq;
   h->filled = false;
+  h->last = pass_layout(h, sh);  // from the shape, since a replayed graph passes by enqueue_body
 }
-
-// Entry values carry 8x8 block bits above the splat id (k_expand) when the
-// tile is 16 pixels (four blocks) and the ids leave four bits free.
-static bool block_masks(int tile, uint32_t n) { return tile == 16 && n <= (1u << ID_BITS); }
 
 // Enqueues project -> bin -> sort -> raster [-> chain/Adam] for the views
 // whose records were uploaded last.  All sizes the device decides (entry
@@ -648,13 +673,8 @@ static bool block_masks(int tile, uint32_t n) { return tile == 16 && n <= (1u <<
 static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   cudaStream_t s = h->stream;
   const int V = sh.V;
-  uint32_t totalTiles = 0, gridCells = 0;
-  for (int v = 0; v < V; ++v) {
-    const uint32_t tx = ceil_div((uint32_t)sh.w[v], (uint32_t)sh.tile), ty = ceil_div((uint32_t)sh.h[v], (uint32_t)sh.tile);
-    totalTiles += tx * ty;
-    gridCells += (tx + 1) * (ty + 1);
-  }
-  h->lastTotalTiles = totalTiles;
+  const PassLayout layout = pass_layout(h, sh);
+  const uint32_t totalTiles = layout.totalTiles, gridCells = layout.gridCells;
   const DevCam* dcams = h->dParams->cams;
   uint32_t* hist = h->small;
   uint32_t* tileCounter = h->small + 2048;
@@ -671,7 +691,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   }
   const uint64_t items = (uint64_t)sh.n * V;
   const bool cull = sh.cull != 0;
-  const bool masks = block_masks(sh.tile, sh.n);
+  const bool masks = layout.masks;
   uint32_t* nItems = h->small + 2061;
   uint32_t* liveItems = h->small + 2150;
   uint32_t* buckets = h->small + 2080;  // 33 sizes and 33 cursors of the work order
@@ -738,7 +758,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   launch_tile_ranges(ta, totalTiles, fork ? h->side : s);
   if (fork) cudaEventRecord(h->joinEv, h->side);
 
-  // presort of the (view, splat) items by depth: 4 byte digits of the depth
+  // presort of the (view, splat) items by depth: the byte digits of the depth
   // bits, stable from slot order, so equal depths stay in splat order.  Views
   // stay interleaved: the tile sort groups entries by global tile id (which
   // belongs to one view) and keeps this order inside every tile.
@@ -752,7 +772,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   pr.status = h->lbStatus;
   pr.statusWord = statusWord;
   pr.epoch = epoch;
-  pr.passes = 4;
+  pr.passes = PRESORT_PASSES;
   pr.keepKeys = false;
   pr.orPasses = 0x7u;  // depth bytes 0-2 spread across a warp; the top byte (sign, exponent) is shared
   pr.histGrid = (unsigned)h->histGrid;
@@ -793,7 +813,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
 
   // stable sort of the entries by global tile id: at most 4 passes, with
   // histograms and block counters of its own behind the presort's four
-  const int passes = (bits_for(totalTiles ? totalTiles - 1 : 0) + 7) / 8;
+  const int passes = layout.passes;
   RadixSortArgs ra{};
   ra.keys[0] = h->keys[0]; ra.keys[1] = h->keys[1];
   ra.vals[0] = h->vals[0]; ra.vals[1] = h->vals[1];
@@ -810,14 +830,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
   ra.histGrid = (unsigned)h->histGrid;
   ra.sweepGrid = (unsigned)h->sweepGrid;
   launch_radix_sort(ra, s);
-  h->lastPasses = passes;
-  h->lastMasks = masks;
   if (cull) launch_ranges_from_keys(h->keys[passes & 1], totalEntries, totalTiles, h->ranges, buckets, s);
-  // kernels: begin, project, tile counts [+ finish], presort (histogram + passes),
-  // entry counts, scan, entry keys, tile sort (histogram + passes),
-  // [ranges from keys], [work order], raster, [visible lists, chain per view, sum + Adam]
-  h->lastLaunches = (cull ? 3u : 4u) + 1u + (uint32_t)pr.passes + 1u + 1u + 1u + 1u + (uint32_t)passes + (cull ? 1u : 0u) +
-                    (h->o.persistent ? 1u : 0u) + 1u + (sh.chain ? 3u : 0u);
   const uint32_t* sortedIds = h->vals[passes & 1];
 
   const bool persistent = h->o.persistent != 0;
@@ -913,7 +926,7 @@ static int ensure_tstore(gs_trainer* h, const Shape& sh) {
   int rc = begin_pass(h);
   if (!rc) rc = enqueue_body(h, probe, false);
   if (rc) return rc;
-  end_pass(h);
+  end_pass(h, probe);
   uint32_t E = 0;
   GS_CK(cudaMemcpyAsync(&E, h->small + 2057, 4, cudaMemcpyDeviceToHost, h->stream));
   GS_CK(cudaStreamSynchronize(h->stream));
@@ -963,7 +976,7 @@ static int run_shape(gs_trainer* h, const Shape& sh) {
     h->filled = false;
     return rc;
   }
-  end_pass(h);
+  end_pass(h, sh);
   return GS_OK;
 }
 
@@ -1298,9 +1311,9 @@ int gs_debug_binning(gs_trainer* h, uint32_t view, uint32_t* tileCnt, uint32_t* 
   if (nEntries) *nEntries = E;
   if (ids) {
     const uint64_t k = std::min<uint64_t>(cap, E);
-    GS_CK(cudaMemcpyAsync(ids, h->vals[h->lastPasses & 1], k * 4, cudaMemcpyDeviceToHost, h->stream));
+    GS_CK(cudaMemcpyAsync(ids, h->vals[h->last.passes & 1], k * 4, cudaMemcpyDeviceToHost, h->stream));
     GS_CK(cudaStreamSynchronize(h->stream));
-    if (h->lastMasks)
+    if (h->last.masks)
       for (uint64_t i = 0; i < k; ++i) ids[i] &= ID_MASK;
   }
   return GS_OK;
@@ -1605,7 +1618,7 @@ int gs_refine(gs_trainer* h, gs_rng_fn rng, void* ctx, gs_refine_result* out) {
     for (auto& a : h->camActiveSh) a = (float)h->o.shDeg;
   }
   // tile-pressure telemetry over the most recent raster's tiles (trainer.js:779-790)
-  launch_max_u32(h->tileCnt, h->lastTotalTiles, h->rf.counts + 2, s);
+  launch_max_u32(h->tileCnt, h->last.totalTiles, h->rf.counts + 2, s);
   uint32_t maxTile = 0;
   GS_CK(cudaMemcpyAsync(&maxTile, h->rf.counts + 2, 4, cudaMemcpyDeviceToHost, s));
   GS_CK(cudaStreamSynchronize(s));

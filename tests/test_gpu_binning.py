@@ -26,3 +26,27 @@ def test_full_lists_of_uneven_views(tile):
         for v in range(len(sizes)):
             check_view_against_oracle(t, oracle_opts(opts), oracle_cam(metas[v], v, len(sizes), 1), params, sh,
                                       targets, n, view=v)
+
+
+@pytest.mark.parametrize("cull", [1, 0])
+def test_lists_after_replayed_passes(cull):
+    """The lists and counts read back belong to the pass that ran last, also
+    when it replayed a captured graph: the tile size changes between passes,
+    and with it the buffer of the sorted entries (one sort pass at tile 16 and
+    32, two at tile 8) and whether entry values carry block bits (tile 16)."""
+    n = 3000
+    params, sh = scene.uniform_scene(n, seed=9, sh_deg=1)
+    params.reshape(-1, 16)[:, 13] += 2.0  # enough donors for refine
+    cam = scene.ring_cameras(1, 3.0, 0.0, 200, 150)[0]
+    rgb = scene.uniform_target(200, 150, seed=30)
+    t, targets, metas = make(params, sh, [cam], [rgb], dict(shDeg=1, tileCull=cull), radius=1.0)
+    launches = {}
+    for tile in [16, 8, 16, 32, 16, 8, 32, 8, 16]:
+        opts = dict(shDeg=1, tile=tile, tileCull=cull)
+        t.setRasterConfig(tile, 64)
+        gpu_raster(t, [0], 3)
+        g, _, _, _ = check_view_against_oracle(t, oracle_opts(opts), oracle_cam(metas[0], 0, 1, 1), params, sh, targets,
+                                               n)
+        assert launches.setdefault(tile, t._state().lastLaunches) == t._state().lastLaunches
+    assert launches[8] == launches[16] + 1
+    assert t.refine(iter([0.5] * 10**6).__next__)["maxTile"] == g["cnt"].max()
