@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(TILE * TILE, TILE == 16 ? GS_RASTER16_MIN_BLOC
               for (int k = 0; k < 10; ++k) rsum[k] = __reduce_add_sync(FULL, (uint32_t)__float2int_rz(xs[k]));
             } else {
 #pragma unroll
-              for (int k = 0; k < 10; ++k) rsum[k] = __reduce_add_sync(FULL, (uint32_t)fix_scaled(xs[k]));
+              for (int k = 0; k < 10; ++k) rsum[k] = __reduce_add_sync(FULL, c2 ? (uint32_t)fix_scaled(xs[k]) : 0u);
             }
             if (c2) {
               S0 = __fmaf_rn(r1.z, aT, S0);
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(RW_WARPS * 32, BWD ? 5 : 6) k_raster_warp(Rast
           const float2 araw = __fmul2_rn(bc2(r1.y), G);
           const bool c2a = T.x >= 1e-4f && ee.x <= E_CUT && araw.x >= A_MIN;
           const bool c2b = T.y >= 1e-4f && ee.y <= E_CUT && araw.y >= A_MIN;
-          // a pixel that does not composite sees alpha 0: C and T stay exactly as they are
+          // a pixel that does not composite sees alpha 0: T stays exactly as it is, and C does while the colour is finite
           const float2 Gm = make_float2(c2a ? G.x : 0.0f, c2b ? G.y : 0.0f);
           const float2 aw = __fmul2_rn(bc2(r1.y), Gm);
           const float2 am = make_float2(fminf(0.99f, aw.x), fminf(0.99f, aw.y));
@@ -632,6 +632,43 @@ __global__ void __launch_bounds__(RW_WARPS * 32, BWD ? 5 : 6) k_raster_warp(Rast
       __syncwarp();
       if (cntA == 0u) cntA = e - s;
       if (cntB == 0u) cntB = e - s;
+    }
+    // An infinite colour (a model's SH coefficients may hold one) made the sums
+    // of the pixels that do not composite its splat 0 * infinity, a NaN.  Colours
+    // are never negative or NaN, so nothing else makes one: then the block's
+    // colours are summed again, each pixel only over what it composites.
+    const float2 cs = __fadd2_rn(__fadd2_rn(C0, C1), C2);
+    if (__any_sync(FULL, isnan(cs.x + cs.y))) {
+      C0 = C1 = C2 = bc2(0.0f);
+      float2 U = make_float2(inA ? 1.0f : 0.0f, inB ? 1.0f : 0.0f);
+      for (uint32_t base = s; base < min(seenEnd, e); base += 32) {
+        const uint32_t n = (uint32_t)__popc(stage(base + lane < e ? a.ids[base + lane] : 0u, base + lane < e, 0));
+        cp_async_wait<0>();
+        __syncwarp();
+#pragma unroll 1
+        for (uint32_t k = 0; k < n; ++k) {
+          const RenderRec& r = s_rec[wid][0][k].rec;
+          float2 Bdy;
+          const float2 ee = pairExponent2(r.r0, r.r1.x, px - r.r0.x, __fadd2_rn(py, bc2(-r.r0.y)), Bdy);
+          const float2 G = gexp2(make_float2(-ee.x, -ee.y));
+          const float2 araw = __fmul2_rn(bc2(r.r1.y), G);
+          if (U.x >= 1e-4f && ee.x <= E_CUT && araw.x >= A_MIN) {
+            const float alpha = fminf(0.99f, araw.x), ta = U.x * alpha;
+            C0.x = __fmaf_rn(ta, r.r1.z, C0.x);
+            C1.x = __fmaf_rn(ta, r.r1.w, C1.x);
+            C2.x = __fmaf_rn(ta, r.r2.x, C2.x);
+            U.x = U.x * (1.0f - alpha);
+          }
+          if (U.y >= 1e-4f && ee.y <= E_CUT && araw.y >= A_MIN) {
+            const float alpha = fminf(0.99f, araw.y), ta = U.y * alpha;
+            C0.y = __fmaf_rn(ta, r.r1.z, C0.y);
+            C1.y = __fmaf_rn(ta, r.r1.w, C1.y);
+            C2.y = __fmaf_rn(ta, r.r2.x, C2.y);
+            U.y = U.y * (1.0f - alpha);
+          }
+        }
+        __syncwarp();
+      }
     }
     C0 = __fadd2_rn(C0, __fmul2_rn(T, bc2(c.bg[0])));
     C1 = __fadd2_rn(C1, __fmul2_rn(T, bc2(c.bg[1])));
@@ -738,7 +775,7 @@ __global__ void __launch_bounds__(RW_WARPS * 32, BWD ? 5 : 6) k_raster_warp(Rast
     // One composited entry at shared address sr, G the pixels' exponentials (0
     // where a pixel does not composite it).  FAST: every product is finite and
     // within +-1e9, so a pixel with G = 0 or without a target (gC = 0)
-    // contributes zeros without being masked.  Advances Ta and S and returns
+    // contributes zeros, and keeps S, without being masked.  Advances Ta and S and returns
     // the lane's ten integer values.
     auto backward = [&](uint32_t sr, float2 G, auto FAST, int32_t q[10]) {
       const float4 r0 = lds4(sr);
@@ -780,11 +817,16 @@ __global__ void __launch_bounds__(RW_WARPS * 32, BWD ? 5 : 6) k_raster_warp(Rast
           !__all_sync(FULL, fabsf(gal16.x) < 1.0e7f && fabsf(gal16.y) < 1.0e7f && gMax < 9.0e8f)) {
 #pragma unroll
         for (int k = 0; k < 10; ++k)
-          xs[k] = make_float2(fminf(fmaxf(xs[k].x, -1.0e9f), 1.0e9f), fminf(fmaxf(xs[k].y, -1.0e9f), 1.0e9f));
+          xs[k] = make_float2(useA ? fminf(fmaxf(xs[k].x, -1.0e9f), 1.0e9f) : 0.0f,
+                              useB ? fminf(fmaxf(xs[k].y, -1.0e9f), 1.0e9f) : 0.0f);
       }
-      S0 = __ffma2_rn(bc2(r1.z), aT, S0);
-      S1 = __ffma2_rn(bc2(r1.w), aT, S1);
-      S2 = __ffma2_rn(bc2(r2.x), aT, S2);
+      const bool setA = decltype(FAST)::value || G.x > 0.0f, setB = decltype(FAST)::value || G.y > 0.0f;
+      const float2 n0 = __ffma2_rn(bc2(r1.z), aT, S0);
+      const float2 n1 = __ffma2_rn(bc2(r1.w), aT, S1);
+      const float2 n2 = __ffma2_rn(bc2(r2.x), aT, S2);
+      S0 = make_float2(setA ? n0.x : S0.x, setB ? n0.y : S0.y);
+      S1 = make_float2(setA ? n1.x : S1.x, setB ? n1.y : S1.y);
+      S2 = make_float2(setA ? n2.x : S2.x, setB ? n2.y : S2.y);
       Ta = Tb;
 #pragma unroll
       for (int k = 0; k < 10; ++k) q[k] = __float2int_rz(xs[k].x) + __float2int_rz(xs[k].y);

@@ -8,7 +8,9 @@ import numpy as np
 import pytest
 
 from splat_b200 import scene
-from test_gpu_parity import check_view_against_oracle, deep_tile_scene, gpu_raster, make, oracle_cam, oracle_opts
+from oracle import oracle as O
+from test_gpu_parity import (assert_bits, check_view_against_oracle, deep_tile_scene, gpu_raster, gpu_view, make,
+                             oracle_cam, oracle_opts)
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +37,45 @@ def test_warp_raster_bitexact(tile, persistent, bright):
     check = make(params, sh, [cam], [rgb.reshape(-1)], dict(opts, tile=16), radius=1.0)[0]
     a, b = t.renderTrainCam(0), check.renderTrainCam(0)
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("tile", [8, 16, 32])
+def test_infinite_colours_stay_where_they_composite(tile, variant):
+    """A model may hold SH coefficients that are infinite, or so large that
+    their sum is: a pixel that does not composite such a splat keeps its
+    colour, and its gradients, in every part of the backward (cached entries
+    and those past the cache, with pixels whose own loss is infinite beside
+    finite ones).  The oracle visits only what a pixel composites."""
+    W, H, n = 75, 53, 4000
+    params, cam = deep_tile_scene(n, seed=4, W=W, H=H)
+    P = params.reshape(-1, 16)
+    rng = np.random.default_rng(tile)
+    P[:, 0] = rng.uniform(-0.8, 0.8, n)  # wider and larger: no pixel composites more than a part of them
+    P[:, 1] = rng.uniform(-0.5, 0.5, n)
+    P[:, 3:6] += 0.8
+    P[:, 13] += 0.7
+    sh = rng.normal(0.0, 0.05, n * 9).astype(np.float32)
+    wild = rng.choice(n, 24, replace=False)
+    sh.reshape(n, 9)[wild[:8], ::4] = np.inf
+    sh.reshape(n, 9)[wild[8:16], :] = rng.choice([-3.0e38, 3.0e38], (8, 9))
+    sh.reshape(n, 9)[wild[16:], 0] = np.nan  # a colour of NaN is 0
+    rgb = scene.uniform_target(W, H, seed=6).reshape(H, W, 3)
+    rgb[rng.random((H, W)) < 0.1] = -1.0
+    opts = dict(shDeg=1, tile=tile, backwardVariant=variant)
+    t, targets, metas = make(params, sh, [cam], [rgb.reshape(-1)], opts, radius=1.0)
+    o, c = oracle_opts(opts), oracle_cam(metas[0], 0, 1, 1)
+    proj = O.project(o, c, params, sh, n)
+    b = O.bin_tiles(o, c, proj, n)
+    r = O.render(o, c, proj, b, targets, n, train=True, ncams=1, variant=variant)
+    img = np.asarray(r["img"]).reshape(H, W, 4)
+    bad = np.isinf(img[..., :3]).any(-1)
+    assert 0.01 < bad.mean() < 0.5 and not np.isnan(img).any()
+    assert np.asarray(r["end"]).max() > 300  # past the 256 entries a warp's cache holds
+    gpu_raster(t, [0], 3)
+    g = gpu_view(t, 0, metas[0], n, tile=tile)
+    assert_bits(g["img"], r["img"], "image")
+    assert_bits(g["finalT"], r["finalT"], "final transmittance")
+    assert_bits(g["end"], r["end"], "end indices")
+    assert_bits(g["gradP"], r["gradP"].reshape(-1, 16)[:, :10], "fixed-point screen-space gradients")
+    assert_bits(t.renderTrainCam(0).reshape(-1), r["img"], "forward-only image")
