@@ -335,7 +335,7 @@ def run_ours(args):
         t.iter = 2000
 
     restore()
-    # ---- autotuner: tile size x splat-batch depth on the first batch ----
+    # ---- autotuner: tile size on the first batch (the depth matters to the stored-state variant only) ----
     tune_tile, tune_depth, tune_table = t.autotune(batch_cams(0), reps=2)
     # ---- plain per-view step (the reference's stepOnce) ----
     restore()

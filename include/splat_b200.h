@@ -277,8 +277,10 @@ GS_API int gs_sort_entries_static(uint32_t* keys, uint32_t* vals, uint32_t n, ui
  * on it: images and gradients are identical for every tile size and depth,
  * only the per-tile entry lists follow the tile size) ----
  * gs_autotune times the training pass on views ci[0..nviews) for each tile
- * edge {8, 16, 32} x splat-batch depth {64, 128, 256}, keeps the fastest
- * and reports it; msOut (9 floats, tile-major) may be NULL. */
+ * edge {8, 16, 32} and, in the stored-state variant, each splat-batch depth
+ * {64, 128, 256}, keeps the fastest and reports it; without that variant the
+ * depth stays as it is and a tile's three times are one.  msOut (9 floats,
+ * tile-major) may be NULL. */
 GS_API int gs_autotune(gs_trainer* h, const uint32_t* ci, uint32_t nviews, int32_t reps, int32_t* bestTile,
                        int32_t* bestDepth, float* msOut);
 GS_API int gs_set_raster_config(gs_trainer* h, int32_t tile, int32_t batchDepth);

@@ -47,7 +47,7 @@ struct Shape {
   int grads;      // write gradF/shGrad readout
   int variant;
   int tile;       // raster tile edge
-  int depth;      // splat-batch depth
+  int depth;      // splat-batch depth (stored-state variant, else 0)
   int cull;       // tile lists culled by the ellipse/tile test
   bool operator<(const Shape& o) const { return std::memcmp(this, &o, sizeof(Shape)) < 0; }
 };
@@ -1021,7 +1021,7 @@ static Shape make_shape(gs_trainer* h, const DevCam* views, int V, int mode, int
   sh.grads = grads;
   sh.variant = h->o.backwardVariant;
   sh.tile = h->tile;
-  sh.depth = h->o.batchDepth;
+  sh.depth = sh.variant == 1 ? h->o.batchDepth : 0;  // nothing else depends on it
   sh.cull = h->o.tileCull;
   return sh;
 }
@@ -1354,9 +1354,11 @@ int gs_debug_gradp(gs_trainer* h, uint32_t view, int32_t* gradP10, int32_t clear
 }
 
 // Autotuner: times the training pass (raster + chain, parameters untouched)
-// on views ci[0..nviews) for every tile edge {8, 16, 32} x splat-batch depth
-// {64, 128, 256} and keeps the fastest.  Loss statistics and camera
-// gradients accumulated meanwhile are restored.
+// on views ci[0..nviews) for every tile edge {8, 16, 32} and, in the
+// stored-state variant, every splat-batch depth {64, 128, 256}, and keeps the
+// fastest.  Without that variant no kernel depends on the depth: each tile is
+// timed once and the depth stays.  Loss statistics and camera gradients
+// accumulated meanwhile are restored.
 int gs_autotune(gs_trainer* h, const uint32_t* ci, uint32_t nv, int32_t reps, int32_t* bestTile, int32_t* bestDepth,
                 float* msOut) {
   if (!h) return GS_E_INVALID;
@@ -1373,13 +1375,14 @@ int gs_autotune(gs_trainer* h, const uint32_t* ci, uint32_t nv, int32_t reps, in
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  const int tiles[3] = {8, 16, 32}, depths[3] = {64, 128, 256};
+  const bool sweep = h->o.backwardVariant == 1;
+  const int tiles[3] = {8, 16, 32}, depths[3] = {64, 128, 256}, nd = sweep ? 3 : 1;
   float best = 3.0e38f;
   int bt = h->tile, bd = h->o.batchDepth;
   for (int ti = 0; ti < 3 && rc == GS_OK; ++ti)
-    for (int di = 0; di < 3 && rc == GS_OK; ++di) {
+    for (int di = 0; di < nd && rc == GS_OK; ++di) {
       h->tile = tiles[ti];
-      h->o.batchDepth = depths[di];
+      if (sweep) h->o.batchDepth = depths[di];
       DevCam views[MAXB];
       for (uint32_t k = 0; k < nv; ++k)
         views[k] = make_cam(h, h->cams[ci[k]], 1, h->camOffset[ci[k]], ci[k], h->camActiveSh[ci[k]]);
@@ -1394,8 +1397,9 @@ int gs_autotune(gs_trainer* h, const uint32_t* ci, uint32_t nv, int32_t reps, in
       float ms = 0.0f;
       cudaEventElapsedTime(&ms, e0, e1);
       ms /= (float)reps;
-      if (msOut) msOut[ti * 3 + di] = ms;
-      if (ms < best) { best = ms; bt = tiles[ti]; bd = depths[di]; }
+      if (msOut)
+        for (int d = di; d < (sweep ? di + 1 : 3); ++d) msOut[ti * 3 + d] = ms;
+      if (ms < best) { best = ms; bt = tiles[ti]; bd = h->o.batchDepth; }
     }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);

@@ -373,8 +373,9 @@ class GSTrainer:
 
     # ---- raster configuration ----
     def autotune(self, cams=None, reps=3):
-        """Pick tile size {8,16,32} x splat-batch depth {64,128,256} by timing
-        the training pass on `cams` (default: the first few cameras).
+        """Pick the tile size {8,16,32} -- and the splat-batch depth {64,128,256}
+        where the stored-state variant uses one -- by timing the training pass
+        on `cams` (default: the first few cameras).
         Returns (tile, depth, {(tile, depth): ms})."""
         if cams is None:
             cams = list(range(min(len(self.camMeta), int(self._o.maxBatch))))

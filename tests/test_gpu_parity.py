@@ -444,6 +444,28 @@ def test_autotune_picks_a_config_and_keeps_results():
     assert_bits(st1, st0, "stats after autotune")
 
 
+@pytest.mark.parametrize("variant", [0, 1])
+def test_autotune_sweeps_the_depth_where_it_matters(variant):
+    """Only the stored-state raster stages entries at the batch depth: without
+    it each tile is timed once, its three times are one and the caller's depth
+    stays; the steps after it equal those of a handle that was not tuned."""
+    params, sh, cams, rgbs = config0(n=3000, seed=7)
+    opts = dict(shDeg=2, batchDepth=128, backwardVariant=variant)
+    t, _, _ = make(params, sh, cams, rgbs, opts, radius=1.0)
+    u, _, _ = make(params, sh, cams, rgbs, opts, radius=1.0)
+    tile, depth, table = t.autotune([0], reps=2)
+    rows = [[table[(ti, d)] for d in (64, 128, 256)] for ti in (8, 16, 32)]
+    assert min(table.values()) == table[(tile, depth)]
+    if variant == 0:
+        assert depth == 128 and all(len(set(r)) == 1 for r in rows), table
+    else:
+        assert any(len(set(r)) > 1 for r in rows), table
+    for h in (t, u):
+        h.setRasterConfig(tile, 64)
+        h.stepBatch([0])
+    assert_bits(t.readGaussians()["data"], u.readGaussians()["data"], "params after a tuned and an untuned step")
+
+
 def test_tile_cull_changes_no_training_result():
     """Three batched steps with culled and with full tile lists: parameters,
     moments and loss statistics bit-identical; fewer entries when culled."""
