@@ -385,8 +385,8 @@ __device__ __forceinline__ uint32_t band_columns(const float4 cq, float mx, floa
   if (!bandIntervalMask(cq, Y0, Y0 + 7.0f, xl, xr)) return 1u;
   const float sl = 4.0e-6f * (fabsf(mx) + fmaxf(fabsf(xl), fabsf(xr)) + 8.0f);
   const int base = 2 * (int)ca;
-  const int l = min(max(__float2int_ru(fminf(((xl + mx) - 7.5f - sl) * 0.125f, 1.0e9f)) - base, 0), 65535);
-  const int r = min(__float2int_rd(fmaxf(((xr + mx) - 0.5f + sl) * 0.125f, -1.0e9f)) - base, 65535);
+  const int l = min(max(__float2int_ru(fminf(fmaxf(((xl + mx) - 7.5f - sl) * 0.125f, -1.0e9f), 1.0e9f)) - base, 0), 65535);
+  const int r = min(__float2int_rd(fminf(fmaxf(((xr + mx) - 0.5f + sl) * 0.125f, -1.0e9f), 1.0e9f)) - base, 65535);
   if (r < 0) return 1u;
   return (uint32_t)l | ((uint32_t)r << 16);
 }

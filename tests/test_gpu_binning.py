@@ -50,3 +50,31 @@ def test_lists_after_replayed_passes(cull):
         assert launches.setdefault(tile, t._state().lastLaunches) == t._state().lastLaunches
     assert launches[8] == launches[16] + 1
     assert t.refine(iter([0.5] * 10**6).__next__)["maxTile"] == g["cnt"].max()
+
+
+@pytest.mark.parametrize("budget", [0, 1])
+def test_splats_billions_of_pixels_wide(budget):
+    """Splats right of the image that reach more than 2^34 pixels to the left:
+    every block column between is theirs, with the whole rows that the usual
+    expansion writes and with the lane's own walk after a tile went over the
+    entry budget."""
+    W, H, n = 150, 70, 40
+    rng = np.random.default_rng(12)
+    f, z = 3.0e6, 0.06
+    P = np.zeros((n, 16), np.float32)
+    P[:, 0] = (rng.uniform(100.0, 130.0, n)) * z / f  # mean 25 to 55 pixels right of the image
+    P[:, 1] = rng.uniform(-40.0, 40.0, n) * z / f
+    P[:, 2] = z + 1.0e-3 * np.arange(n)
+    P[:, 3:6] = [5.9, -12.0, -12.0]  # 1.8e10 by 307 pixels (sigma)
+    P[:, 6] = 1.0
+    P[:, 10:13] = rng.normal(0.0, 1.0, (n, 3))
+    P[:, 13] = -2.0
+    cam = dict(R=[1, 0, 0, 0, 1, 0, 0, 0, 1], t=[0, 0, 0], f=f, cx=W / 2, cy=H / 2, w=W, h=H)
+    params, sh = P.reshape(-1), np.zeros(n * 9, np.float32)
+    opts = dict(shDeg=1, **(dict(entriesCap=700) if budget else {}))
+    t, targets, metas = make(params, sh, [cam], [scene.uniform_target(W, H, seed=5)], opts, radius=1.0)
+    gpu_raster(t, [0], 3)
+    g, _, _, b = check_view_against_oracle(t, oracle_opts(opts), oracle_cam(metas[0], 0, 1, 1), params, sh, targets, n)
+    x0 = g["rect"][0::2] & 0xFFFF
+    assert (x0[g["rect"][0::2] != 0xFFFFFFFF] > 0).any() and (g["img"].reshape(H, W, 4)[:16, 64:, 3] > 0.5).all()
+    assert b["dropped"].any() == bool(budget)
