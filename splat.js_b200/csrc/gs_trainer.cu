@@ -361,6 +361,8 @@ int gs_setup(gs_trainer* h, const float* params, uint32_t n, const float* sh, co
   cudaSetDevice(h->device);
   cudaStreamSynchronize(h->stream);
   free_all(h);
+  h->lastV = 0;  // no raster of this set-up yet: the buffers may be smaller than the last one's
+  h->last = {};
   const gs_options& o = h->o;
   h->n = n;
   // cap (trainer.js:105-107)
