@@ -154,10 +154,9 @@ constexpr uint32_t ID_BITS = 28;
 constexpr uint32_t ID_MASK = (1u << ID_BITS) - 1u;
 
 constexpr int RW_WARPS = 4;                    // warps per block of k_raster_warp
-#ifndef GS_RASTER_CACHE
-#define GS_RASTER_CACHE 256  // composited entries a warp caches (k_raster_warp)
-#endif
-constexpr uint32_t RASTER_CACHE_ENTRIES = GS_RASTER_CACHE;
+// composited entries a warp caches (k_raster_warp): in an allocation of its own,
+// and at most, where the memory is there anyway
+constexpr uint32_t RASTER_CACHE_ENTRIES = 256, RASTER_CACHE_MAX = 1024;
 
 // Work-order bucket of a tile: 32 empty, 0 longest.
 __device__ __forceinline__ uint32_t tile_bucket(uint2 r) { return (uint32_t)__clz((int)(r.y - r.x)); }

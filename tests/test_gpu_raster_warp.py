@@ -16,8 +16,9 @@ pytestmark = pytest.mark.gpu
 
 
 # budget 60000: the entries' buffers cannot hold the cache, which gets its own
-# allocation of 256 entries a block; 0 (12M entries): it lies in the buffers
-@pytest.mark.parametrize("budget", [0, 60000])
+# allocation of 256 entries a warp; 768000: it lies in the buffers, 247 deep;
+# 0 (12M entries): there, 1024 deep
+@pytest.mark.parametrize("budget", [0, 60000, 768000])
 @pytest.mark.parametrize("bright", [0, 1])
 @pytest.mark.parametrize("persistent", [0, 1])
 @pytest.mark.parametrize("tile", [8, 16, 32])
