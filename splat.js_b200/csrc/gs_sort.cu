@@ -1,20 +1,23 @@
-// gs_sort.cu -- global sorted binning: exclusive scan of per-splat entry
-// counts, and a onesweep LSD radix sort (8-bit digits, decoupled look-back)
-// of the (globalTile << 32 | depth bits, splat id) entries.
+// gs_sort.cu -- exclusive scans of entry and flag counts, and a onesweep LSD
+// radix sort (8-bit digits, decoupled look-back)
+// of (key, value) pairs: items by depth bits, entries by global tile id,
+// refine's donors by size.
 //
 // The reference bins with atomic per-tile cursors and sorts each tile segment
 // with a bitonic network (shaders.js:378-500); its final order is, per tile,
-// ascending (depth f32 bits, id).  Here every entry is keyed by
-// (tile, depth) and written in splat order, so one stable sort over all
-// entries leaves each tile's ids in exactly that order.
+// ascending (depth f32 bits, id).  Here the splats are sorted by depth (stable,
+// in id order), expanded into entries in that order, and the entries sorted by
+// tile (stable), which leaves each tile's ids in exactly that order.
 //
 // Onesweep: one histogram kernel reads every key once and counts all digit
 // positions; each digit pass then ranks a block of entries in shared memory
 // (warp ballots give each key its rank among equal digits), publishes the
 // block's per-digit counts, and obtains the count of every earlier block by
-// decoupled look-back before scattering.  Blocks are claimed in order through
-// an atomic counter by a grid that is entirely resident, so every block it
-// waits on is already running.  Each spin has an iteration limit; on expiry
+// decoupled look-back before scattering.  Blocks of entries are claimed in
+// order through an atomic counter by thread blocks that are running, so every
+// block waited on was claimed by one that runs too, whatever else is on the
+// device (in a captured step the tile counts run beside the presort, and not
+// all of the grid need be resident).  Each spin has an iteration limit; on expiry
 // the kernel sets ST_LOOKBACK_TIMEOUT in the status word and carries on.
 //
 // Look-back status words are 64-bit: [63:32] epoch tag, [31:30] flag,
@@ -291,7 +294,7 @@ __device__ __forceinline__ void onesweep_body(const OnesweepArgs& a, OnesweepSha
     if (tile >= numTiles) break;
     const uint32_t base = tile * RS_TILE;
 
-    // load: warp w holds entries [base + w*512, +512), item j at lane l
+    // load: warp w holds 32 * RS_ITEMS entries in order, item j at lane l
     KT key[RS_ITEMS];
     uint32_t val[RS_ITEMS];
     uint32_t dig[RS_ITEMS];
@@ -524,7 +527,7 @@ int onesweep_grid(int device) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per64, k_onesweep<uint64_t>, RS_THREADS, rs_dyn_smem<uint64_t>());
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perOr, k_onesweep<uint32_t, false, true>, RS_THREADS,
                                                 rs_dyn_smem<uint32_t>());
-  int perSm = per32 < per64 ? per32 : per64;  // one grid size that is fully resident for every form
+  int perSm = per32 < per64 ? per32 : per64;  // one grid size that fills the device alone, for every form
   if (perOr < perSm) perSm = perOr;
   if (perSm < 1) perSm = 1;
   return sms * perSm;

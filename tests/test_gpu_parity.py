@@ -93,7 +93,7 @@ def assert_bits(a, b, what):
                           f"{a.reshape(-1)[bad[:5]]} vs {b.reshape(-1)[bad[:5]]}"
 
 
-def check_view_against_oracle(t, o, ocam, params, sh, targets, n, view=0):
+def check_view_against_oracle(t, o, ocam, params, sh, targets, n, view=0, variant=0):
     g = gpu_view(t, view, dict(w=ocam.w, h=ocam.h), n, tile=o.tile)
     proj = O.project(o, ocam, params, sh if o.shDeg else None, n)
     rec, rect = O.records(o, ocam, proj, n)
@@ -106,7 +106,7 @@ def check_view_against_oracle(t, o, ocam, params, sh, targets, n, view=0):
     assert_bits(g["ranges"][:, 0] - base, b["start"][:-1], "tile starts")
     assert_bits(g["ranges"][:, 1] - base, b["start"][1:], "tile ends")
     assert_bits(g["ids"][base:base + len(b["ids"])], b["ids"], "per-tile ordered ids (sort permutation)")
-    r = O.render(o, ocam, proj, b, targets, n, train=True, ncams=ocam.ncams)
+    r = O.render(o, ocam, proj, b, targets, n, train=True, ncams=ocam.ncams, variant=variant)
     assert_bits(g["img"], r["img"], "image")
     assert_bits(g["finalT"], r["finalT"], "final transmittance")
     assert_bits(g["end"], r["end"], "end indices")
@@ -168,14 +168,14 @@ def oracle_adam(t, iter_after, radius, horizon=60000, opacityReg=0.01, shLr=1.25
                      float(np.float32(math.log(radius * 0.05))), reg=opacityReg, shLr=shLr)
 
 
-@pytest.mark.parametrize("cull,depth,persistent", [(1, 64, 1), (0, 64, 1), (1, 128, 1), (1, 256, 1), (1, 256, 0)])
-def test_config0_raster_bitexact(cull, depth, persistent):
+@pytest.mark.parametrize("cull,persistent", [(1, 1), (0, 1), (1, 0), (0, 0)])
+def test_config0_raster_bitexact(cull, persistent):
     """cull=0: the reference's full rectangle lists, per-tile order included;
-    depth: entries staged per shared-memory batch of the fused raster;
-    persistent=0: one block per tile instead of the persistent work queue."""
+    persistent=0: a block per four 8x8 pixel blocks instead of the persistent
+    work queue."""
     params, sh, cams, rgbs = config0()
     n = len(params) // 16
-    opts = dict(shDeg=2, tileCull=cull, batchDepth=depth, persistent=persistent)
+    opts = dict(shDeg=2, tileCull=cull, persistent=persistent)
     t, targets, metas = make(params, sh, cams, rgbs, opts, radius=1.0)
     gpu_raster(t, [0], 3)
     check_view_against_oracle(t, oracle_opts(opts), oracle_cam(metas[0], 0, 1, 2), params, sh, targets, n)
@@ -512,8 +512,8 @@ def test_needles_and_discs_bitexact(tile):
 
 def deep_tile_scene(n, seed=0, W=64, H=64):
     """n small, faint splats crowded over one 16x16 tile: its list holds far
-    more than 4096 entries (past the rasteriser's ballot-bit capacity and
-    over many shared-memory batches) while no pixel saturates."""
+    more than 4096 entries (past the stored-state raster's ballot-bit capacity
+    and over many shared-memory batches) while no pixel saturates."""
     rng = np.random.default_rng(seed)
     P = np.zeros((n, 16), np.float32)
     # tile (2, 2) of a 64x64 view at f = 64, z = 3: world x, y in [0, 0.75)
@@ -530,18 +530,20 @@ def deep_tile_scene(n, seed=0, W=64, H=64):
     return P.reshape(-1), cam
 
 
-@pytest.mark.parametrize("depth", [64, 256])
-def test_deep_tile_bitexact(depth):
-    """A tile list past 4096 entries: the backward walks those entries without
-    ballot bits; images, lists and gradients must still match the oracle."""
+@pytest.mark.parametrize("variant,depth", [(0, 64), (1, 64), (1, 128), (1, 256)])
+def test_deep_tile_bitexact(variant, depth):
+    """A tile list past 4096 entries: the warps' exponential caches are full
+    long before, and the stored-state variant (at every depth of its
+    shared-memory batches) walks those entries without ballot bits; images,
+    lists and gradients must still match the oracle."""
     n = 9000
     params, cam = deep_tile_scene(n)
     sh = np.zeros(n * 3 * 8, np.float32)
-    opts = dict(shDeg=2, batchDepth=depth)
+    opts = dict(shDeg=2, batchDepth=depth, backwardVariant=variant)
     t, targets, metas = make(params, sh, [cam], [scene.uniform_target(64, 64, seed=5)], opts, radius=1.0)
     gpu_raster(t, [0], 3)
     g, r, proj, b = check_view_against_oracle(t, oracle_opts(opts), oracle_cam(metas[0], 0, 1, 2), params, sh,
-                                              targets, n)
+                                              targets, n, variant=variant)
     assert np.diff(b["start"]).max() > 4096      # a list past the bit capacity
     assert np.asarray(r["end"]).max() > 4096     # and pixels that composite past it
 
