@@ -41,9 +41,9 @@ METRIC = "train views/s @1M splats 1080p, batched vs plain step, 1 B200, grads w
 FLOP_PER_PAIR = 26 + 70   # raster forward + backward per evaluated pixel-entry pair (FFMA = 2)
 # DRAM bytes (read + write) of one raster launch over an 8-view batch at the
 # default workload: one ncu capture of a 2-view launch of the same scene
-# (two 1080p ring views; 1193.39 MB read + 1696.07 MB written, most of it the
+# (two 1080p ring views; 1241.39 MB read + 1729.15 MB written, most of it the
 # exponential cache), scaled by the view count (not measured live)
-RASTER_DRAM_BYTES_8VIEW = (1193.393e6 + 1696.066e6) * 4
+RASTER_DRAM_BYTES_8VIEW = (1241.393e6 + 1729.145e6) * 4
 
 
 def parse():

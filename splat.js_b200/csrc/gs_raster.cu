@@ -472,12 +472,12 @@ struct StagedRec {
 // slower where a few long blocks decide the time (an evaluation pass, one
 // 1080p view: 6830 -> 6506 us; 555x419, 180k splats: 7009 -> 6376 us).
 //
-// What bounds it: instruction issue (67% active), with the conversions to
-// integers (F2I: 8 cycles a warp) at 55% of their pipe and FMA at 57%.  Measured
-// on 1M splats, two 1080p views: 2.04 ms, 1.56 G warp instructions; the block
+// What bounds it: instruction issue (69% active), with the conversions to
+// integers (F2I: 8 cycles a warp) at 56% of their pipe and FMA at 60%.  Measured
+// on 1M splats, two 1080p views: 2.01 ms, 1.57 G warp instructions; the block
 // per tile of four warps it replaced, which met at a barrier every batch and
-// recomputed G: 2.49 ms, 2.08 G.  The cache's traffic goes through DRAM (2.9 GB
-// in that pass, 1.4 TB/s), loaded two entries ahead; without the cache a train
+// recomputed G: 2.49 ms, 2.08 G.  The cache's traffic goes through DRAM (3.0 GB
+// in that pass, 1.5 TB/s), loaded two entries ahead; without the cache a train
 // step is 7% slower.
 template <int TILE, bool MASKED, bool BWD>
 __global__ void __launch_bounds__(RW_WARPS * 32, BWD ? 5 : 6) k_raster_warp(RasterArgs a) {
