@@ -274,8 +274,9 @@ __device__ __forceinline__ float adam_g(float g) { return fabsf(g) < 1e18f ? g :
 // slot and camera gradients are integer sums, so no result depends on it.
 // A block takes PER strips of 256 splats: the atomics of all blocks go to the
 // views' counters, one cache sector, one after another, and with one strip
-// they were the whole time (42 us for 8 views of 1M splats); below 256k splats
-// one strip spreads the work over more SMs.
+// they were the whole time (42 us for 8 views of 1M splats, 19 with eight);
+// below 400k items one strip spreads the work over more SMs.  One / eight strips,
+// us: 262k items 2.9 / 3.8, 400k 4.2 / 4.0, 480k (8 views of 60k) 4.5 / 4.0.
 template <int PER>
 __global__ void __launch_bounds__(256) k_visible_list(ChainArgs a, uint32_t blocksPerView) {
   __shared__ uint32_t s_warp[8 * PER];
@@ -557,10 +558,12 @@ void launch_chain_adam(const ChainArgs& args, int deg, cudaStream_t s) {
   ChainArgs a = args;
   const unsigned blocks = (a.n + 127) / 128;
   if (blocks == 0) return;
-  // strips per chain block: four while that leaves 16 blocks per SM
-  a.chainStrips = (uint64_t)blocks * a.V >= 4ull * 16 * 148 ? 4 : 1;
+  // strips per chain block: four while that leaves 16 blocks per SM.  One / four
+  // strips, us: 1.04M items (8 views) 67.0 / 68.7, 1.4M (2 views) 89.5 / 84.1,
+  // 8M 494 / 450; 120k 12.5 / 18.9
+  a.chainStrips = (uint64_t)blocks * a.V >= 4ull * 16 * a.sms ? 4 : 1;
   const unsigned g1 = (blocks + a.chainStrips - 1) / a.chainStrips * (unsigned)a.V;
-  if (a.n >= (1u << 18)) {
+  if ((uint64_t)a.n * a.V >= 400000u) {
     const unsigned bpv = (a.n + 2047) / 2048;
     k_visible_list<8><<<bpv * (unsigned)a.V, 256, 0, s>>>(a, bpv);
   } else {

@@ -26,6 +26,7 @@ struct StepBeginArgs {
   uint32_t items;
   uint32_t* clear[3];      // word ranges set to zero
   uint32_t count[3];
+  uint32_t sms;            // of the device
 };
 
 struct ProjectArgs {
@@ -209,6 +210,7 @@ struct ChainArgs {
   uint32_t* visList;       // V * n: per view, indices of the visible splats
   uint32_t* visCount;      // V counters, cleared before the step
   uint32_t chainStrips;    // strips of 128 list items per chain block (set by the launcher)
+  uint32_t sms;            // of the device
   float anisoReg;
   int32_t* gradCam;
   float* gradF;            // optional readout (n * 16)

@@ -728,8 +728,8 @@ __global__ void __launch_bounds__(256) k_ranges_from_keys(const uint32_t* keys, 
 void launch_step_begin(const StepBeginArgs& a, cudaStream_t s) {
   uint32_t words = 0;
   for (int r = 0; r < 3; ++r) words = a.count[r] > words ? a.count[r] : words;
-  const unsigned blocks = (words + 1023) / 1024;  // clearing, four words a thread
-  k_step_begin<<<1 + (blocks < 296 ? (blocks ? blocks : 1) : 296), 256, 0, s>>>(a);
+  const unsigned blocks = (words + 1023) / 1024, most = 2 * a.sms;  // clearing, four words a thread
+  k_step_begin<<<1 + (blocks < most ? (blocks ? blocks : 1) : most), 256, 0, s>>>(a);
 }
 void launch_project(const ProjectArgs& a, int deg, cudaStream_t s) {
   const unsigned grid = (a.n + PROJECT_THREADS - 1) / PROJECT_THREADS;

@@ -722,6 +722,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
     ba.count[1] = 2057;
     ba.clear[2] = h->small + 2062;  // visible-item counters, work order, live items
     ba.count[2] = 2151 - 2062;
+    ba.sms = (uint32_t)h->sms;
     launch_step_begin(ba, s);
   }
 
@@ -909,6 +910,7 @@ static int enqueue_body(gs_trainer* h, const Shape& sh, bool fork) {
     c.v = h->v;
     c.shM = h->shM;
     c.shV = h->shV;
+    c.sms = (uint32_t)h->sms;
     launch_chain_adam(c, h->o.shDeg, s);
   }
   if (h->profiling) {
